@@ -727,7 +727,11 @@ rt_status rt_trace_host(rt_scene* scene, const RtRay* h_rays, uint32_t n, RtHit*
   }();
   const uint32_t growth = kGrowth ? kGrowth : (direct ? 8u : 4u);
   const uint32_t chunk = std::min<uint32_t>(n, direct ? (1u << 24) : (1u << 23));  // buffer capacity
-  const size_t ray_bytes = (size_t)chunk * sizeof(RtRay), hit_bytes = direct ? 0 : (size_t)chunk * sizeof(RtHit);
+  // each half's rays and hits start 256-byte aligned: straight after an odd number of 8-byte hits the second
+  // half's rays would be off the 16 bytes that the kernels load them by
+  auto up256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t ray_bytes = up256((size_t)chunk * sizeof(RtRay));
+  const size_t hit_bytes = direct ? 0 : up256((size_t)chunk * sizeof(RtHit));
   const size_t per = ray_bytes + hit_bytes;
   const size_t need = 2 * per;
   cudaError_t e;

@@ -141,6 +141,14 @@ def test_trace_host_matches_device(rt, cuda):
     assert np.array_equal(f.view(np.uint64), h.view(np.uint64))
 
 
+@pytest.mark.parametrize("n", [1, 524_289, 700_001, 3_000_003])
+def test_trace_host_odd_counts(rt, cuda, n):
+    """An odd count that takes two staging chunks: both halves of the staging buffer are aligned."""
+    rays = rt.gen_rays(14, 0, n, 1.0, 1e-4, float("inf"))
+    with rt.Scene(rt.gen_soup(14, 0, 3_000, 1.0, 0.01)) as sc:
+        assert np.array_equal(sc.trace_host(rays).view(np.uint64), dev_trace(rt, cuda, sc, rays).view(np.uint64))
+
+
 def test_caller_supplied_nodes(rt, orc, cuda):
     tris, ubo, rays = rt.gen_config1()
     nodes, _, _, _ = orc.build_bvh(tris, mode=1)
