@@ -26,9 +26,7 @@ void set_error(const std::string& msg);
 
 namespace {
 
-constexpr int kT = 256;            // threads per block
-constexpr int kItems = 16;         // keys per thread in the sort tiles
-constexpr int kTile = kT * kItems;  // 4096 keys per tile
+constexpr int kT = 256;  // threads per block
 constexpr int kBins = 256;
 
 __device__ __forceinline__ uint32_t f2ord(float f) {  // order-preserving float -> uint
@@ -99,7 +97,7 @@ __device__ __forceinline__ uint32_t spread3(uint32_t v) {
 }
 
 __global__ void k_morton(const RtTriangle64* tris, const RtSphere32* sph, uint32_t nt, uint32_t n, const float* box,
-                         uint32_t mode, uint32_t* codes, uint32_t* idx) {
+                         uint32_t mode, uint32_t* codes) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float c[3];
@@ -111,123 +109,157 @@ __global__ void k_morton(const RtTriangle64* tris, const RtSphere32* sph, uint32
     q[k] = f2u_sat(off * 1024.0f);
   }
   codes[i] = (spread3(q[2]) << 2) | (spread3(q[1]) << 1) | spread3(q[0]);
-  idx[i] = i;
 }
 
 // ---- stable LSD radix sort, 8-bit digits ----
-// hist layout: [bin][tile], so an exclusive scan in that order gives each
-// (bin, tile) its output base.
-__global__ void __launch_bounds__(kT) k_rs_hist(const uint32_t* keys, uint32_t n, uint32_t shift, uint32_t* hist,
-                                                uint32_t tiles) {
+// A tile is 256 x ITEMS keys.  Per pass: k_rs_hist counts each tile's digits
+// ([bin][tile]), k_rs_scan turns each bin's row into exclusive offsets (one
+// block a bin) and leaves the bin's total, and k_rs_scatter adds the totals of
+// lower bins, ranks its keys and writes them.  Bound by latency below about
+// 10^5 keys and by L2 above (keys and indices of 4 M primitives, 67 MB with
+// both copies, stay in L2).  The scan took 182 us a pass at 4,194,304 keys as
+// one block over all 262,144 counts.  Whole build, before and after: 1,860 ->
+// 1,094 us at 4,194,304 primitives, 187 -> 124 us at 20,482.
+constexpr int kItemsLarge = 16;  // 4096-key tiles: 64-byte runs per digit on average
+constexpr int kItemsSmall = 4;   // 1024-key tiles: four times the blocks
+// Tiles of kItemsSmall up to here: at 1 M keys the large tiles are down to 256
+// blocks, under two per SM.
+constexpr uint32_t kSmallSort = 1u << 20;
+
+constexpr uint32_t tile_keys(uint32_t n) { return kT * (n <= kSmallSort ? kItemsSmall : kItemsLarge); }
+
+__global__ void __launch_bounds__(kT) k_rs_hist(const uint32_t* __restrict__ keys, uint32_t n, uint32_t shift,
+                                                uint32_t* __restrict__ hist, uint32_t tiles, uint32_t tile) {
   __shared__ uint32_t h[kBins];
   h[threadIdx.x] = 0u;
   __syncthreads();
-  const uint32_t base = blockIdx.x * kTile;
-  for (int j = 0; j < kItems; ++j) {
-    const uint32_t i = base + j * kT + threadIdx.x;
-    if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
-  }
+  const uint32_t base = blockIdx.x * tile;
+#pragma unroll 4
+  for (uint32_t j = threadIdx.x; j < tile; j += kT)
+    if (base + j < n) atomicAdd(&h[(keys[base + j] >> shift) & 255u], 1u);
   __syncthreads();
   hist[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// Exclusive scan of `len` counts in place, one block of 1024 threads, in
-// chunks of 8192: each thread sums 8 consecutive counts, a warp scan with
-// __shfl_up_sync and a scan of the 32 warp totals give each thread its
-// starting offset, and a running carry links the chunks.  (Loads of
-// consecutive threads stay within the same sectors; a thread-per-stretch
-// serial scan made every load of a warp touch 32 lines.)
-__global__ void __launch_bounds__(1024) k_scan_inplace(uint32_t* a, uint32_t len) {
-  __shared__ uint32_t warp_sums[32];
-  const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
-  uint32_t carry = 0;
-  for (uint32_t base = 0; base < len; base += 8192u) {
-    const uint32_t i0 = base + 8u * t;
-    uint32_t v[8], sum = 0;
+// Exclusive scan of x over the block's kT threads; *total gets the sum.
+__device__ __forceinline__ uint32_t block_scan(uint32_t x, uint32_t* warp_sums, uint32_t* total) {
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  uint32_t v = x;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      v[k] = i0 + k < len ? a[i0 + k] : 0u;
-      sum += v[k];
-    }
-    uint32_t x = sum;  // inclusive scan over the warp
-#pragma unroll
-    for (uint32_t off = 1; off < 32; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
-      if (lane >= off) x += y;
-    }
-    if (lane == 31u) warp_sums[w] = x;
-    __syncthreads();
-    if (w == 0) {
-      uint32_t z = warp_sums[lane];
-#pragma unroll
-      for (uint32_t off = 1; off < 32; off <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, z, off);
-        if (lane >= off) z += y;
-      }
-      warp_sums[lane] = z;  // inclusive prefix of the warp totals
-    }
-    __syncthreads();
-    uint32_t run = carry + (w ? warp_sums[w - 1] : 0u) + x - sum;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (i0 + k < len) a[i0 + k] = run;
-      run += v[k];
-    }
-    carry += warp_sums[31];
-    __syncthreads();  // warp_sums is rewritten by the next chunk
+  for (uint32_t off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, off);
+    if (lane >= off) v += y;
   }
+  if (lane == 31u) warp_sums[w] = v;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kT / 32; ++k) {
+    const uint32_t c = warp_sums[k];
+    before += k < w ? c : 0u;
+    all += c;
+  }
+  __syncthreads();  // warp_sums may be rewritten
+  *total = all;
+  return before + v - x;
 }
 
-// Each warp owns a contiguous 512-key stretch of the tile and walks it in
-// order, 32 keys at a time; equal digits within a step are ranked by lane
-// (__match_any_sync), and per-warp running counts keep earlier steps ahead.
-__global__ void __launch_bounds__(kT) k_rs_scatter(const uint32_t* keys, const uint32_t* vals, uint32_t n,
-                                                   uint32_t shift, const uint32_t* offs, uint32_t tiles,
-                                                   uint32_t* keys_out, uint32_t* vals_out) {
-  constexpr int kWarps = kT / 32;
-  constexpr int kPerWarp = kTile / kWarps;  // 512
+// Block b: exclusive scan of bin b's tile counts in place, its total to totals[b].
+__global__ void __launch_bounds__(kT) k_rs_scan(uint32_t* __restrict__ hist, uint32_t tiles,
+                                                uint32_t* __restrict__ totals) {
+  __shared__ uint32_t warp_sums[kT / 32];
+  uint32_t* row = hist + (size_t)blockIdx.x * tiles;
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < tiles; base += 4u * kT) {
+    const uint32_t i0 = base + 4u * threadIdx.x;
+    uint32_t v[4], sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = i0 + k < tiles ? row[i0 + k] : 0u;
+      sum += v[k];
+    }
+    uint32_t run = carry + block_scan(sum, warp_sums, &total);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i0 + k < tiles) row[i0 + k] = run;
+      run += v[k];
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
+// Each warp holds a contiguous stretch of 32 x ITEMS keys of the tile and ranks
+// it in order, 32 keys at a time: equal digits within a step rank by lane
+// (__match_any_sync), a per-warp count keeps earlier steps ahead.  The tile is
+// put in digit order in shared memory first, so that a digit's keys leave as
+// one run of consecutive addresses.  vals == nullptr: the value is the index
+// (the first pass).
+template <int ITEMS>
+__global__ void __launch_bounds__(kT) k_rs_scatter(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+                                                   uint32_t n, uint32_t shift, const uint32_t* __restrict__ offs,
+                                                   const uint32_t* __restrict__ totals, uint32_t tiles,
+                                                   uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
+  constexpr int kWarps = kT / 32, kTile = kT * ITEMS;
   __shared__ uint32_t cnt[kWarps][kBins];
-  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  for (int b = lane; b < kBins; b += 32) cnt[w][b] = 0u;
-  __syncwarp();
-  const uint32_t base = blockIdx.x * kTile + w * kPerWarp;
-  // pass 1: this warp's digit counts
-  for (int s = 0; s < kPerWarp; s += 32) {
-    const uint32_t i = base + s + lane;
-    const bool ok = i < n;
-    const uint32_t d = ok ? (keys[i] >> shift) & 255u : 256u;
+  __shared__ uint32_t sk[kTile], sv[kTile];
+  __shared__ uint32_t to[kBins];  // output position of the digit's first key less its position in the tile
+  __shared__ uint32_t warp_sums[kWarps];
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, b = threadIdx.x;  // kT == kBins
+  for (int i = lane; i < kBins; i += 32) cnt[w][i] = 0u;
+  const uint32_t base = blockIdx.x * kTile, first = base + w * 32u * ITEMS + lane;
+  const uint32_t live = min((uint32_t)kTile, n - base);
+  uint32_t k[ITEMS], v[ITEMS], rank[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t i = first + 32u * j;
+    k[j] = i < n ? keys[i] : 0u;
+    v[j] = i < n && vals ? vals[i] : i;
+  }
+  uint32_t all;
+  const uint32_t bin_base = block_scan(totals[b], warp_sums, &all) + offs[b * tiles + blockIdx.x];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const bool ok = first + 32u * j < n;
+    const uint32_t d = ok ? (k[j] >> shift) & 255u : 256u;
     const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-    if (ok && lane == (uint32_t)(__ffs(peers) - 1)) cnt[w][d] += (uint32_t)__popc(peers);
+    const uint32_t seen = ok ? cnt[w][d] : 0u;
+    rank[j] = seen + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+    __syncwarp();
+    if (ok && lane == (uint32_t)(__ffs(peers) - 1)) cnt[w][d] = seen + (uint32_t)__popc(peers);
     __syncwarp();
   }
   __syncthreads();
-  // per bin: global base of this tile + counts of earlier warps
-  {
-    const uint32_t b = threadIdx.x;  // kT == kBins
-    uint32_t run = offs[b * tiles + blockIdx.x];
+  {  // per digit: the warps' counts become offsets within the digit, then within the tile
+    uint32_t run = 0;
+#pragma unroll
     for (int ww = 0; ww < kWarps; ++ww) {
       const uint32_t c = cnt[ww][b];
       cnt[ww][b] = run;
       run += c;
     }
+    const uint32_t start = block_scan(run, warp_sums, &all);
+#pragma unroll
+    for (int ww = 0; ww < kWarps; ++ww) cnt[ww][b] += start;
+    to[b] = bin_base - start;
   }
   __syncthreads();
-  // pass 2: place keys in order
-  for (int s = 0; s < kPerWarp; s += 32) {
-    const uint32_t i = base + s + lane;
-    const bool ok = i < n;
-    const uint32_t k = ok ? keys[i] : 0u;
-    const uint32_t d = ok ? (k >> shift) & 255u : 256u;
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-    const uint32_t lt = peers & ((1u << lane) - 1u);
-    if (ok) {
-      const uint32_t pos = cnt[w][d] + (uint32_t)__popc(lt);
-      keys_out[pos] = k;
-      vals_out[pos] = vals[i];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j)
+    if (first + 32u * j < n) {
+      const uint32_t at = cnt[w][(k[j] >> shift) & 255u] + rank[j];
+      sk[at] = k[j];
+      sv[at] = v[j];
     }
-    __syncwarp();
-    if (ok && lane == (uint32_t)(__ffs(peers) - 1)) cnt[w][d] += (uint32_t)__popc(peers);
-    __syncwarp();
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t i = j * kT + threadIdx.x;
+    if (i < live) {
+      const uint32_t key = sk[i], pos = to[(key >> shift) & 255u] + i;
+      keys_out[pos] = key;
+      vals_out[pos] = sv[i];
+    }
   }
 }
 
@@ -349,8 +381,8 @@ __global__ void k_bottom_up(uint32_t N, RtBVHNode40* nodes, const uint32_t* pare
 }  // namespace
 
 size_t device_build_scratch_bytes(uint32_t n) {
-  const uint32_t tiles = (n + kTile - 1) / kTile;
-  return 256 + (size_t)n * 4 * 4 + (size_t)kBins * tiles * 4 + (size_t)(2 * (size_t)n) * 4 * 2;
+  const uint32_t tiles = (n + tile_keys(n) - 1) / tile_keys(n);
+  return 256 + kBins * 4 + (size_t)n * 4 * 4 + (size_t)kBins * tiles * 4 + (size_t)(2 * (size_t)n) * 4 * 2;
 }
 
 // nodes: 2n-1 records; scratch: device_build_scratch_bytes(n).
@@ -362,6 +394,8 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
   uint32_t* ordbox = reinterpret_cast<uint32_t*>(p);
   float* box = reinterpret_cast<float*>(p + 64);
   p += 256;
+  uint32_t* totals = reinterpret_cast<uint32_t*>(p);
+  p += kBins * 4;
   uint32_t* ka = reinterpret_cast<uint32_t*>(p);
   p += (size_t)n * 4;
   uint32_t* va = reinterpret_cast<uint32_t*>(p);
@@ -370,7 +404,7 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
   p += (size_t)n * 4;
   uint32_t* vb = reinterpret_cast<uint32_t*>(p);
   p += (size_t)n * 4;
-  const uint32_t tiles = (n + kTile - 1) / kTile;
+  const uint32_t tile = tile_keys(n), tiles = (n + tile - 1) / tile;
   uint32_t* hist = reinterpret_cast<uint32_t*>(p);
   p += (size_t)kBins * tiles * 4;
   uint32_t* parent = reinterpret_cast<uint32_t*>(p);
@@ -383,13 +417,17 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
   const uint32_t gb = (n + kT - 1) / kT;
   k_centroid_box<<<std::min<uint32_t>(gb, 1024u), kT, 0, st>>>(tris, sph, nt, n, ordbox);
   k_pad_box<<<1, 1, 0, st>>>(ordbox, box);
-  k_morton<<<gb, kT, 0, st>>>(tris, sph, nt, n, box, mode, ka, va);
+  k_morton<<<gb, kT, 0, st>>>(tris, sph, nt, n, box, mode, ka);
   uint32_t *kin = ka, *vin = va, *kout = kb, *vout = vb;
   for (int pass = 0; pass < 4; ++pass) {
     const uint32_t shift = 8u * (uint32_t)pass;
-    k_rs_hist<<<tiles, kT, 0, st>>>(kin, n, shift, hist, tiles);
-    k_scan_inplace<<<1, 1024, 0, st>>>(hist, kBins * tiles);
-    k_rs_scatter<<<tiles, kT, 0, st>>>(kin, vin, n, shift, hist, tiles, kout, vout);
+    const uint32_t* v = pass ? vin : nullptr;
+    k_rs_hist<<<tiles, kT, 0, st>>>(kin, n, shift, hist, tiles, tile);
+    k_rs_scan<<<kBins, kT, 0, st>>>(hist, tiles, totals);
+    if (tile == kT * kItemsSmall)
+      k_rs_scatter<kItemsSmall><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
+    else
+      k_rs_scatter<kItemsLarge><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
     std::swap(kin, kout);
     std::swap(vin, vout);
   }

@@ -73,3 +73,13 @@ def test_device_build_matches_oracle(rt, orc, cuda, mode):
     big = rt.gen_soup(3, 0, 4_194_304, 1.0, 0.002)
     assert np.array_equal(device_build(rt, cuda, big, mode=mode).view(np.uint8),
                           orc.build_bvh(big, mode=mode)[0].view(np.uint8))
+
+
+@pytest.mark.parametrize("n", [1024, 1025, 1_048_576, 1_048_577, 1_052_673])
+def test_device_build_sort_tiles(rt, cuda, n):
+    """Sizes at the edges of the radix sort's tiles and where its tile size changes, for scattered codes and
+    for a few long runs of equal ones."""
+    soup = rt.gen_soup(9, 0, n, 1.0, 0.004)
+    assert np.array_equal(device_build(rt, cuda, soup).view(np.uint8), rt.build_bvh(soup).view(np.uint8))
+    runs = soup[np.arange(n) * 7 // n]
+    assert np.array_equal(device_build(rt, cuda, runs).view(np.uint8), rt.build_bvh(runs).view(np.uint8))
