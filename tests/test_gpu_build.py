@@ -83,3 +83,23 @@ def test_device_build_sort_tiles(rt, cuda, n):
     assert np.array_equal(device_build(rt, cuda, soup).view(np.uint8), rt.build_bvh(soup).view(np.uint8))
     runs = soup[np.arange(n) * 7 // n]
     assert np.array_equal(device_build(rt, cuda, runs).view(np.uint8), rt.build_bvh(runs).view(np.uint8))
+
+
+@pytest.mark.parametrize("n", [511, 512, 513, 1024, 1537, 40_961])
+@pytest.mark.parametrize("shape", ["soup", "equal", "line"])
+def test_device_build_tree_blocks(rt, cuda, n, shape):
+    """Sizes at the edges of the tree kernel's blocks: shallow trees, one code everywhere (the index decides)
+    and a line of clusters (long ranges over many blocks); arrays that are only 4-byte aligned too."""
+    t = rt.gen_soup(11, 0, n, 1.0, 0.01)
+    if shape == "equal":
+        t = np.repeat(t[:1], n)
+    elif shape == "line":
+        for v in ("v0", "v1", "v2"):
+            t[v][:, 0] += (2.0 ** (np.arange(n) % 23)).astype(np.float32)
+    want = rt.build_bvh(t).view(np.uint8)
+    assert np.array_equal(device_build(rt, cuda, t).view(np.uint8), want)
+    raw = cuda.zeros(n * 64 + 4, dtype=cuda.uint8, device="cuda")
+    raw[4:] = cuda.from_numpy(t.view(np.uint8)).cuda()
+    out = cuda.zeros((2 * n - 1) * 40 + 4, dtype=cuda.uint8, device="cuda")
+    rt.build_bvh_device(raw[4:], n, d_nodes=out[4:])
+    assert np.array_equal(out[4:].cpu().numpy(), want)
