@@ -2,11 +2,11 @@
 //
 // Same node layout and the same binary32 operations as the host builder
 // (host_bvh.cpp), so the two emit identical 40-byte node arrays:
-//   k_centroid_box   centroids ((v0+v1)+v2)/3, min/max fold from +-1e9
+//   k_centroids      centroids ((v0+v1)+v2)/3, min/max fold from +-1e9
 //                    (GetEnclosingAABB.comp:64-109); block reduction, then
-//                    atomicMin/Max on order-preserving integer images of floats
-//   k_pad_box        the padding of :105-109, one thread
-//   k_morton         30-bit codes (GenerateMortonCodesOfPrimitives.comp:52-93)
+//                    atomicMax on order-preserving integer images of floats
+//   k_morton         the box's padding (:105-109), 30-bit codes
+//                    (GenerateMortonCodesOfPrimitives.comp:52-93)
 //   radix sort       stable LSD sort of (code, index), 4 passes of 8 bits like
 //                    RadixSortSimple.comp:8-13: per-tile histograms, a scan, and
 //                    a scatter whose ranks keep input order (warp multi-split)
@@ -36,51 +36,96 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-__device__ __forceinline__ void centroid(const RtTriangle64* tris, const RtSphere32* sph, uint32_t nt, uint32_t i,
-                                         float c[3]) {
+// A vertex: one 16-byte load when the caller's array allows it (al16, uniform
+// per launch; the records only promise 4 bytes), else three loads.
+__device__ __forceinline__ void load_vertex(const float* p, bool al16, float v[3]) {
+  if (al16) {
+    const float4 f = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = f.x; v[1] = f.y; v[2] = f.z;
+  } else {
+    v[0] = __ldg(p); v[1] = __ldg(p + 1); v[2] = __ldg(p + 2);
+  }
+}
+
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
+
+__device__ __forceinline__ void centroid(const RtTriangle64* __restrict__ tris, const RtSphere32* __restrict__ sph,
+                                         uint32_t nt, uint32_t i, bool al16, float c[3]) {
   if (i < nt) {
-    const RtTriangle64& t = tris[i];
-    for (int k = 0; k < 3; ++k) c[k] = (t.v0[k] + t.v1[k] + t.v2[k]) / 3.0f;
+    float v0[3], v1[3], v2[3];
+    load_vertex(tris[i].v0, al16, v0);
+    load_vertex(tris[i].v1, al16, v1);
+    load_vertex(tris[i].v2, al16, v2);
+    for (int k = 0; k < 3; ++k) c[k] = (v0[k] + v1[k] + v2[k]) / 3.0f;
   } else {
     const RtSphere32& s = sph[i - nt];
     for (int k = 0; k < 3; ++k) c[k] = s.center[k];
   }
 }
 
-__global__ void k_centroid_box(const RtTriangle64* tris, const RtSphere32* sph, uint32_t nt, uint32_t n,
-                               uint32_t* box /* ord: min xyz, max xyz */) {
+// Centroids, kept for k_morton (12 of a primitive's 64 bytes to read again),
+// and their box: words 0-2 of `box` the complements of the minima's integer
+// images and 3-5 the maxima's, so that both are maxima over words that start at
+// zero.  Bound by HBM: 4,194,304 triangles take 47 us here (6.8 TB/s) and 29 us
+// in k_morton; reading the triangles twice, with scalar loads, took 88 and 72.
+__global__ void __launch_bounds__(kT) k_centroids(const RtTriangle64* __restrict__ tris,
+                                                  const RtSphere32* __restrict__ sph, uint32_t nt, uint32_t n,
+                                                  float* __restrict__ cx, float* __restrict__ cy,
+                                                  float* __restrict__ cz, uint32_t* __restrict__ box) {
+  constexpr int kUnroll = 4;
+  __shared__ float part[6][kT / 32];
+  const bool al16 = aligned16(tris);
   float mn[3] = {1000000000.0f, 1000000000.0f, 1000000000.0f};
   float mx[3] = {-1000000000.0f, -1000000000.0f, -1000000000.0f};
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float c[3];
-    centroid(tris, sph, nt, i, c);
-    for (int k = 0; k < 3; ++k) {
-      mn[k] = fminf(mn[k], c[k]);
-      mx[k] = fmaxf(mx[k], c[k]);
+  for (uint32_t b = blockIdx.x * (kT * kUnroll); b < n; b += gridDim.x * (kT * kUnroll)) {
+    float c[kUnroll][3];
+#pragma unroll
+    for (int j = 0; j < kUnroll; ++j) {
+      const uint32_t i = b + j * kT + threadIdx.x;
+      if (i < n) centroid(tris, sph, nt, i, al16, c[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < kUnroll; ++j) {
+      const uint32_t i = b + j * kT + threadIdx.x;
+      if (i >= n) continue;
+      cx[i] = c[j][0];
+      cy[i] = c[j][1];
+      cz[i] = c[j][2];
+      for (int k = 0; k < 3; ++k) {
+        mn[k] = fminf(mn[k], c[j][k]);
+        mx[k] = fmaxf(mx[k], c[j][k]);
+      }
     }
   }
-  for (int k = 0; k < 3; ++k)
+  for (int k = 0; k < 3; ++k) {
     for (int o = 16; o > 0; o >>= 1) {
       mn[k] = fminf(mn[k], __shfl_down_sync(0xFFFFFFFFu, mn[k], o));
       mx[k] = fmaxf(mx[k], __shfl_down_sync(0xFFFFFFFFu, mx[k], o));
     }
-  if ((threadIdx.x & 31u) == 0)
-    for (int k = 0; k < 3; ++k) {
-      atomicMin(&box[k], f2ord(mn[k]));
-      atomicMax(&box[3 + k], f2ord(mx[k]));
+    if ((threadIdx.x & 31u) == 0u) {
+      part[k][threadIdx.x >> 5] = mn[k];
+      part[3 + k][threadIdx.x >> 5] = mx[k];
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < 6u) {
+    float v = part[threadIdx.x][0];
+    for (int w = 1; w < kT / 32; ++w)
+      v = threadIdx.x < 3u ? fminf(v, part[threadIdx.x][w]) : fmaxf(v, part[threadIdx.x][w]);
+    atomicMax(&box[threadIdx.x], threadIdx.x < 3u ? ~f2ord(v) : f2ord(v));
+  }
 }
 
-__global__ void k_pad_box(const uint32_t* ordbox, float* box) {
+// The padding of GetEnclosingAABB.comp:105-109.
+__device__ __forceinline__ void padded_box(const uint32_t* box, float mn[3], float mx[3]) {
   const float delta = 0.001f, padding = delta / 2.0f;
   for (int k = 0; k < 3; ++k) {
-    float mn = ord2f(ordbox[k]), mx = ord2f(ordbox[3 + k]);
-    if (mx - mn < delta) {
-      mn -= padding;
-      mx += padding;
+    mn[k] = ord2f(~box[k]);
+    mx[k] = ord2f(box[3 + k]);
+    if (mx[k] - mn[k] < delta) {
+      mn[k] -= padding;
+      mx[k] += padding;
     }
-    box[k] = mn;
-    box[3 + k] = mx;
   }
 }
 
@@ -95,19 +140,40 @@ __device__ __forceinline__ uint32_t spread3(uint32_t v) {
   return v;
 }
 
-__global__ void k_morton(const RtTriangle64* tris, const RtSphere32* sph, uint32_t nt, uint32_t n, const float* box,
-                         uint32_t mode, uint32_t* codes) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float c[3];
-  centroid(tris, sph, nt, i, c);
+__device__ __forceinline__ uint32_t morton(const float c[3], const float mn[3], const float mx[3], uint32_t mode) {
   uint32_t q[3];
   for (int k = 0; k < 3; ++k) {
-    const float span = box[3 + k] - box[k];
-    const float off = mode == RT_BVH_REFERENCE ? c[k] / span : (c[k] - box[k]) / span;
+    const float span = mx[k] - mn[k];
+    const float off = mode == RT_BVH_REFERENCE ? c[k] / span : (c[k] - mn[k]) / span;
     q[k] = f2u_sat(off * 1024.0f);
   }
-  codes[i] = (spread3(q[2]) << 2) | (spread3(q[1]) << 1) | spread3(q[0]);
+  return (spread3(q[2]) << 2) | (spread3(q[1]) << 1) | spread3(q[0]);
+}
+
+// Codes of one sort tile and their digit counts for the sort's first pass.
+__global__ void __launch_bounds__(kT) k_morton(const float* __restrict__ cx, const float* __restrict__ cy,
+                                               const float* __restrict__ cz, uint32_t n,
+                                               const uint32_t* __restrict__ box, uint32_t mode,
+                                               uint32_t* __restrict__ codes, uint32_t* __restrict__ hist,
+                                               uint32_t tiles, uint32_t tile) {
+  __shared__ uint32_t h[kBins];
+  h[threadIdx.x] = 0u;
+  float mn[3], mx[3];
+  padded_box(box, mn, mx);
+  __syncthreads();
+  const uint32_t base = blockIdx.x * tile;
+#pragma unroll 4
+  for (uint32_t j = threadIdx.x; j < tile; j += kT) {
+    const uint32_t i = base + j;
+    if (i < n) {
+      const float c[3] = {cx[i], cy[i], cz[i]};
+      const uint32_t code = morton(c, mn, mx, mode);
+      codes[i] = code;
+      atomicAdd(&h[code & 255u], 1u);
+    }
+  }
+  __syncthreads();
+  hist[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
 // ---- stable LSD radix sort, 8-bit digits ----
@@ -116,9 +182,9 @@ __global__ void k_morton(const RtTriangle64* tris, const RtSphere32* sph, uint32
 // block a bin) and leaves the bin's total, and k_rs_scatter adds the totals of
 // lower bins, ranks its keys and writes them.  Bound by latency below about
 // 10^5 keys and by L2 above (keys and indices of 4 M primitives, 67 MB with
-// both copies, stay in L2).  The scan took 182 us a pass at 4,194,304 keys as
-// one block over all 262,144 counts.  Whole build, before and after: 1,860 ->
-// 1,094 us at 4,194,304 primitives, 187 -> 124 us at 20,482.
+// both copies, stay in L2).  us per pass at 4,194,304 keys, before and now: hist
+// 11 / 7, scan 182 / 3.5 (it was one block over all 262,144 counts), scatter 91 /
+// 40 (50 with __match_any_sync, which stalled the warps, or at 127 registers).
 constexpr int kItemsLarge = 16;  // 4096-key tiles: 64-byte runs per digit on average
 constexpr int kItemsSmall = 4;   // 1024-key tiles: four times the blocks
 // Tiles of kItemsSmall up to here: at 1 M keys the large tiles are down to 256
@@ -133,9 +199,19 @@ __global__ void __launch_bounds__(kT) k_rs_hist(const uint32_t* __restrict__ key
   h[threadIdx.x] = 0u;
   __syncthreads();
   const uint32_t base = blockIdx.x * tile;
+  if (base + tile <= n) {  // tiles start 16-byte aligned
+    const uint4* k4 = reinterpret_cast<const uint4*>(keys + base);
 #pragma unroll 4
-  for (uint32_t j = threadIdx.x; j < tile; j += kT)
-    if (base + j < n) atomicAdd(&h[(keys[base + j] >> shift) & 255u], 1u);
+    for (uint32_t j = threadIdx.x; j < tile / 4u; j += kT) {
+      const uint4 k = k4[j];
+      atomicAdd(&h[(k.x >> shift) & 255u], 1u);
+      atomicAdd(&h[(k.y >> shift) & 255u], 1u);
+      atomicAdd(&h[(k.z >> shift) & 255u], 1u);
+      atomicAdd(&h[(k.w >> shift) & 255u], 1u);
+    }
+  } else {
+    for (uint32_t i = base + threadIdx.x; i < n; i += kT) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
+  }
   __syncthreads();
   hist[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
@@ -190,12 +266,12 @@ __global__ void __launch_bounds__(kT) k_rs_scan(uint32_t* __restrict__ hist, uin
 
 // Each warp holds a contiguous stretch of 32 x ITEMS keys of the tile and ranks
 // it in order, 32 keys at a time: equal digits within a step rank by lane
-// (__match_any_sync), a per-warp count keeps earlier steps ahead.  The tile is
+// (a ballot per digit bit), a per-warp count keeps earlier steps ahead.  The tile is
 // put in digit order in shared memory first, so that a digit's keys leave as
 // one run of consecutive addresses.  vals == nullptr: the value is the index
 // (the first pass).
 template <int ITEMS>
-__global__ void __launch_bounds__(kT) k_rs_scatter(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+__global__ void __launch_bounds__(kT, 4) k_rs_scatter(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                                                    uint32_t n, uint32_t shift, const uint32_t* __restrict__ offs,
                                                    const uint32_t* __restrict__ totals, uint32_t tiles,
                                                    uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
@@ -208,20 +284,25 @@ __global__ void __launch_bounds__(kT) k_rs_scatter(const uint32_t* __restrict__ 
   for (int i = lane; i < kBins; i += 32) cnt[w][i] = 0u;
   const uint32_t base = blockIdx.x * kTile, first = base + w * 32u * ITEMS + lane;
   const uint32_t live = min((uint32_t)kTile, n - base);
-  uint32_t k[ITEMS], v[ITEMS], rank[ITEMS];
+  uint32_t k[ITEMS], rank[ITEMS];
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const uint32_t i = first + 32u * j;
     k[j] = i < n ? keys[i] : 0u;
-    v[j] = i < n && vals ? vals[i] : i;
   }
   uint32_t all;
   const uint32_t bin_base = block_scan(totals[b], warp_sums, &all) + offs[b * tiles + blockIdx.x];
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const bool ok = first + 32u * j < n;
-    const uint32_t d = ok ? (k[j] >> shift) & 255u : 256u;
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+    const uint32_t d = (k[j] >> shift) & 255u;
+    uint32_t peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const bool one = (d >> b) & 1u;
+      const uint32_t ones = __ballot_sync(0xFFFFFFFFu, one);
+      peers &= one ? ones : ~ones;
+    }
     const uint32_t seen = ok ? cnt[w][d] : 0u;
     rank[j] = seen + (uint32_t)__popc(peers & ((1u << lane) - 1u));
     __syncwarp();
@@ -248,7 +329,7 @@ __global__ void __launch_bounds__(kT) k_rs_scatter(const uint32_t* __restrict__ 
     if (first + 32u * j < n) {
       const uint32_t at = cnt[w][(k[j] >> shift) & 255u] + rank[j];
       sk[at] = k[j];
-      sv[at] = v[j];
+      sv[at] = vals ? vals[first + 32u * j] : first + 32u * j;
     }
   __syncthreads();
 #pragma unroll
@@ -267,17 +348,6 @@ __device__ __forceinline__ void pad_axis(float& mn, float& mx) {
   if (mx - mn < delta) {
     mn -= padding;
     mx += padding;
-  }
-}
-
-// A vertex: one 16-byte load when the caller's array allows it (al16, uniform
-// per launch; the records only promise 4 bytes), else three loads.
-__device__ __forceinline__ void load_vertex(const float* p, bool al16, float v[3]) {
-  if (al16) {
-    const float4 f = __ldg(reinterpret_cast<const float4*>(p));
-    v[0] = f.x; v[1] = f.y; v[2] = f.z;
-  } else {
-    v[0] = __ldg(p); v[1] = __ldg(p + 1); v[2] = __ldg(p + 2);
   }
 }
 
@@ -330,118 +400,148 @@ __device__ __forceinline__ int delta_next(const uint32_t* __restrict__ codes, ui
 // records; climbing on in k_tree itself kept whole blocks resident for one
 // thread's chain of atomics.  The two replace a leaf pass, a pass of Karras
 // searches and a bottom-up pass with a global atomic and two 40-byte record
-// reads per node.  Whole build of 4,194,304 triangles: 1,094 us before, 948 us
-// with the climb inside k_tree, 808 us with k_top, 760 us with the climb cut
-// in two (k_tree alone 311 -> 262 us, bound by issue and by the gather: 518 MB
-// read and 289 MB written at 3 TB/s; k_top 67 us of serial atomics).
+// reads per node.  4,194,304 triangles: 666 us for those three; k_tree 311 us as
+// one climb per thread, 260 with the climb cut in two, 195 with 8-byte stores,
+// padded rows and one box array (bound by issue; 518 MB read, most of it the
+// gather, and 289 MB written); k_top 65 us of serial atomics.
 constexpr int kLeaves = 512;
 constexpr int kFirstClimb = 4;
 constexpr uint32_t kRight = 0x8000u;  // shared slot: the visitor was the right child
+// Row of the boxes in shared memory: leaves, then internal nodes; five words of
+// padding keep the ten words of neighbouring records in different banks.
+constexpr int kBoxRow = 2 * kLeaves + 5;
+constexpr uint32_t kLinked = 0x80000000u, kLeafLeft = 0x10000u, kLeafRight = 0x20000u;
 
 __global__ void __launch_bounds__(kLeaves) k_tree(const RtTriangle64* __restrict__ tris,
                                                   const RtSphere32* __restrict__ sph, uint32_t nt, uint32_t n,
                                                   uint32_t mode, const uint32_t* __restrict__ codes,
                                                   const uint32_t* __restrict__ order, RtBVHNode40* __restrict__ nodes,
                                                   uint2* __restrict__ open, uint32_t* __restrict__ num_open) {
-  __shared__ float leaf[6][kLeaves], inner[6][kLeaves];
-  __shared__ uint32_t left_of[kLeaves], right_of[kLeaves];  // links of internal node base + i (0 and 0: not here)
+  // positions are relative to the block's first leaf
+  __shared__ float bx[6][kBoxRow];
+  __shared__ uint32_t link[kLeaves];   // internal node: its split | kLeafLeft | kLeafRight | kLinked (0: not here)
   __shared__ uint32_t prim[kLeaves];
-  __shared__ uint32_t slot[kLeaves];   // split after base + i: 0, or a visitor's far end + 1 (and kRight)
-  __shared__ uint32_t climb[kLeaves];  // nodes to climb on from: l - base | (r - base) << 16
-  __shared__ int8_t gap[kLeaves + 1];  // delta of base + i - 1 and base + i
+  __shared__ uint32_t slot[kLeaves];   // split after i: 0, or a visitor's far end + 1 (and kRight)
+  __shared__ uint32_t climb[kLeaves];  // nodes to climb on from: l | r << 16
+  __shared__ int8_t gap[kLeaves + 1];  // delta of i - 1 and i; -1 at the ends of the whole order
   __shared__ uint32_t num_climb, num_edge, num_lone, open_at;
   __shared__ uint2 edge[2];
   const uint32_t t = threadIdx.x, base = blockIdx.x * kLeaves, i0 = base + t;
-  const uint32_t leaf_off = n - 1u;
+  const uint32_t live = min((uint32_t)kLeaves, n - base);
   slot[t] = 0u;
-  left_of[t] = right_of[t] = 0u;
-  if (i0 < n) gap[t] = i0 > 0u ? (int8_t)delta_next(codes, i0 - 1u) : (int8_t)-1;
+  link[t] = 0u;
+  if (t <= live) gap[t] = i0 > 0u && i0 < n ? (int8_t)delta_next(codes, i0 - 1u) : (int8_t)-1;
   if (t == 0u) {
-    gap[kLeaves] = base + kLeaves < n ? (int8_t)delta_next(codes, base + kLeaves - 1u) : (int8_t)-1;
+    if (live == kLeaves) gap[kLeaves] = base + kLeaves < n ? (int8_t)delta_next(codes, base + kLeaves - 1u) : (int8_t)-1;
     num_climb = num_edge = num_lone = 0u;
   }
   float box[6];
-  if (i0 < n) {
+  if (t < live) {
     const uint32_t g = mode == RT_BVH_REFERENCE ? i0 : order[i0];
-    leaf_box(tris, sph, nt, g, (reinterpret_cast<uintptr_t>(tris) & 15u) == 0u, box);
+    leaf_box(tris, sph, nt, g, aligned16(tris), box);
     prim[t] = g;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) leaf[k][t] = box[k];
+    for (int k = 0; k < 6; ++k) bx[k][t] = box[k];
   }
   __syncthreads();
   // Half of the climbers stop at every level, and a warp climbs as long as its
   // last lane: after kFirstClimb levels the rest move together into few warps.
-  uint32_t l = i0, r = i0;
-  bool climbing = i0 < n && n > 1u;
+  uint32_t l = t, r = t;
+  int gl = 0, gr = 0;  // the gaps before l and after r
+  bool climbing = t < live && n > 1u;
+  if (climbing) {
+    gl = gap[t];
+    gr = gap[t + 1u];
+  }
   for (int part = 0; part < 2; ++part) {
     if (part == 1) {
       __syncthreads();
-      if (climbing) climb[atomicAdd(&num_climb, 1u)] = (l - base) | (r - base) << 16;
+      if (climbing) climb[atomicAdd(&num_climb, 1u)] = l | r << 16;
       __syncthreads();
       climbing = t < num_climb;
       if (!climbing) break;
-      const uint32_t c = climb[t];
-      l = base + (c & 0xFFFFu);
-      r = base + (c >> 16);
-      const bool is_left = l == 0u || (r != n - 1u && gap[r + 1u - base] > gap[l - base]);
+      l = climb[t] & 0xFFFFu;
+      r = climb[t] >> 16;
+      gl = gap[l];
+      gr = gap[r + 1u];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) box[k] = inner[k][(is_left ? r : l) - base];
+      for (int k = 0; k < 6; ++k) box[k] = bx[k][kLeaves + (gr > gl ? r : l)];
     }
     for (int step = 0; climbing && (part == 1 || step < kFirstClimb); ++step) {
-      const bool is_left = l == 0u || (r != n - 1u && gap[r + 1u - base] > gap[l - base]);
+      const bool is_left = gr > gl;
       const uint32_t s = is_left ? r : l - 1u;  // the parent's split
       climbing = false;
-      if (is_left ? s + 1u >= base + kLeaves : l == base) {  // its other child is in another block
-        edge[atomicAdd(&num_edge, 1u)] = make_uint2(l, r);   // one node at each edge at most
+      if (is_left ? r == kLeaves - 1u : l == 0u) {  // its other child is in another block
+        edge[atomicAdd(&num_edge, 1u)] = make_uint2(base + l, base + r);  // one node at each edge at most
         break;
       }
       __threadfence_block();
-      const uint32_t other = atomicExch(&slot[s - base], is_left ? l - base + 1u : (r - base + 1u) | kRight);
+      const uint32_t other = atomicExch(&slot[s], is_left ? l + 1u : (r + 1u) | kRight);
       if (other == 0u) break;
       __threadfence_block();
-      slot[s - base] = 0u;  // both children have met
-      const uint32_t end = base + (other & (kRight - 1u)) - 1u;
-      if (is_left) r = end;
-      else l = end;
-      const bool leaf_l = l == s, leaf_r = s + 1u == r;
-      const uint32_t sib = is_left ? (leaf_r ? r : s + 1u) - base : s - base;
-      if (is_left ? leaf_r : leaf_l) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) box[k] = (k & 1) ? fmaxf(box[k], leaf[k][sib]) : fminf(box[k], leaf[k][sib]);
+      slot[s] = 0u;  // both children have met
+      const uint32_t end = (other & (kRight - 1u)) - 1u;
+      uint32_t sib;
+      if (is_left) {
+        sib = end == s + 1u ? end : kLeaves + s + 1u;
+        r = end;
+        gr = gap[end + 1u];
       } else {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) box[k] = (k & 1) ? fmaxf(box[k], inner[k][sib]) : fminf(box[k], inner[k][sib]);
+        sib = end == s ? s : kLeaves + s;
+        l = end;
+        gl = gap[end];
       }
-      const bool root = l == 0u && r == n - 1u;
-      const uint32_t at = root ? 0u : ((l == 0u || (r != n - 1u && gap[r + 1u - base] > gap[l - base])) ? r : l) - base;
+      const bool root = (gl & gr) < 0;
+      const uint32_t at = root ? 0u : (gr > gl ? r : l);  // this node's number
 #pragma unroll
-      for (int k = 0; k < 6; ++k) inner[k][at] = box[k];
-      left_of[at] = leaf_l ? leaf_off + s : s;
-      right_of[at] = leaf_r ? leaf_off + r : s + 1u;
+      for (int k = 0; k < 6; ++k) {
+        const float b = bx[k][sib];
+        box[k] = (k & 1) ? fmaxf(box[k], b) : fminf(box[k], b);
+        bx[k][kLeaves + at] = box[k];
+      }
+      link[at] = s | (l == s ? kLeafLeft : 0u) | (r == s + 1u ? kLeafRight : 0u) | kLinked;
       climbing = !root;
     }
   }
   __syncthreads();
-  {  // the block's records, ten words each, in address order
-    const uint32_t live = min((uint32_t)kLeaves, n - base);
-    uint32_t* out = reinterpret_cast<uint32_t*>(nodes + leaf_off + base);
-    for (uint32_t j = t; j < live * 10u; j += kLeaves) {
-      const uint32_t i = j / 10u, w = j - 10u * i, g = prim[i];
-      uint32_t v = 0u;
-      if (w < 6u) v = __float_as_uint(leaf[w][i]);
-      else if (w == 8u) v = g < nt ? g : g - nt;
-      else if (w == 9u) v = g < nt ? RT_PRIM_TRIANGLE : RT_PRIM_SPHERE;
-      out[j] = v;
-    }
-    out = reinterpret_cast<uint32_t*>(nodes + base);
-    for (uint32_t j = t; j < live * 10u; j += kLeaves) {
-      const uint32_t i = j / 10u, w = j - 10u * i;
-      if (right_of[i] == 0u) continue;  // not an internal node that is complete here
-      uint32_t v = 0u;
-      if (w < 6u) v = __float_as_uint(inner[w][i]);
-      else if (w == 6u) v = left_of[i];
-      else if (w == 7u) v = right_of[i];
-      out[j] = v;
+  {  // the block's records in address order, five 8-byte words each
+    const uint32_t leaf_off = n - 1u;
+    const bool al8 = (reinterpret_cast<uintptr_t>(nodes) & 7u) == 0u;  // the records only promise 4
+    auto put = [&](uint32_t* p, uint32_t x, uint32_t y) {
+      if (al8) {
+        *reinterpret_cast<uint2*>(p) = make_uint2(x, y);
+      } else {
+        p[0] = x;
+        p[1] = y;
+      }
+    };
+    uint32_t* out_leaf = reinterpret_cast<uint32_t*>(nodes + leaf_off + base);
+    uint32_t* out_inner = reinterpret_cast<uint32_t*>(nodes + base);
+    for (uint32_t j = t; j < live * 5u; j += kLeaves) {
+      const uint32_t i = j / 5u, w = j - 5u * i;
+      uint32_t x = 0u, y = 0u;
+      if (w < 3u) {
+        x = __float_as_uint(bx[2u * w][i]);
+        y = __float_as_uint(bx[2u * w + 1u][i]);
+      } else if (w == 4u) {
+        const uint32_t g = prim[i];
+        x = g < nt ? g : g - nt;
+        y = g < nt ? RT_PRIM_TRIANGLE : RT_PRIM_SPHERE;
+      }
+      put(out_leaf + 2u * j, x, y);
+      const uint32_t k = link[i];
+      if (k == 0u) continue;  // not an internal node that is complete here
+      x = y = 0u;
+      if (w < 3u) {
+        x = __float_as_uint(bx[2u * w][kLeaves + i]);
+        y = __float_as_uint(bx[2u * w + 1u][kLeaves + i]);
+      } else if (w == 3u) {
+        x = base + (k & 0xFFFFu);
+        y = x + 1u;
+        if (k & kLeafLeft) x += leaf_off;
+        if (k & kLeafRight) y += leaf_off;
+      }
+      put(out_inner + 2u * j, x, y);
     }
   }
   // The nodes k_top climbs on from: those at the edges and the visitors that
@@ -509,10 +609,14 @@ __global__ void __launch_bounds__(128) k_top(uint32_t n, const uint32_t* __restr
 
 }  // namespace
 
+// Cleared at the start: the centroid box (six words, two unused), the count of
+// k_tree's list, then a slot per split.
+constexpr size_t kClearWords = 9;
+
 size_t device_build_scratch_bytes(uint32_t n) {
   const uint32_t tiles = (n + tile_keys(n) - 1) / tile_keys(n);
   const uint32_t blocks = (n + kLeaves - 1) / kLeaves;
-  return 256 + 8 + kBins * 4 + (size_t)n * 4 * 4 + (size_t)blocks * 8 + (size_t)kBins * tiles * 4 + 4 + (size_t)n * 4;
+  return 16 + kBins * 4 + (size_t)n * 4 * 4 + (size_t)blocks * 8 + (size_t)kBins * tiles * 4 + kClearWords * 4 + (size_t)n * 4;
 }
 
 // nodes: 2n-1 records; scratch: device_build_scratch_bytes(n).
@@ -521,16 +625,13 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
   const uint32_t n = nt + ns;
   if (n == 0) return cudaSuccess;
   char* p = static_cast<char*>(scratch);
-  uint32_t* ordbox = reinterpret_cast<uint32_t*>(p);
-  float* box = reinterpret_cast<float*>(p + 64);
-  p += 256;
   uint32_t* totals = reinterpret_cast<uint32_t*>(p);
   p += kBins * 4;
   uint32_t* ka = reinterpret_cast<uint32_t*>(p);
   p += (size_t)n * 4;
   uint32_t* va = reinterpret_cast<uint32_t*>(p);
   p += (size_t)n * 4;
-  p = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(p) + 7) & ~(uintptr_t)7);
+  p = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
   // k_tree's list takes the sort's second buffers, which four passes leave
   // free: at most one entry per leaf and one more per block
   uint2* open = reinterpret_cast<uint2*>(p);
@@ -543,21 +644,22 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
   const uint32_t tile = tile_keys(n), tiles = (n + tile - 1) / tile;
   uint32_t* hist = reinterpret_cast<uint32_t*>(p);
   p += (size_t)kBins * tiles * 4;
-  uint32_t* num_open = reinterpret_cast<uint32_t*>(p);  // the list's count, then the slots: cleared together
-  uint32_t* slots = num_open + 1;
+  uint32_t* box = reinterpret_cast<uint32_t*>(p);
+  uint32_t *num_open = box + kClearWords - 1, *slots = box + kClearWords;
 
-  uint32_t init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
-  cudaError_t e = cudaMemcpyAsync(ordbox, init, sizeof(init), cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaMemsetAsync(box, 0, (kClearWords + (size_t)n) * 4, st);
   if (e != cudaSuccess) return e;
-  const uint32_t gb = (n + kT - 1) / kT;
-  k_centroid_box<<<std::min<uint32_t>(gb, 1024u), kT, 0, st>>>(tris, sph, nt, n, ordbox);
-  k_pad_box<<<1, 1, 0, st>>>(ordbox, box);
-  k_morton<<<gb, kT, 0, st>>>(tris, sph, nt, n, box, mode, ka);
+  // the centroids take buffers that the sort's first pass does not read
+  float *cx = reinterpret_cast<float*>(va), *cy = reinterpret_cast<float*>(kb), *cz = reinterpret_cast<float*>(vb);
+  const uint32_t sms = (uint32_t)device_sm_count();
+  k_centroids<<<std::min<uint32_t>((n + kT * 4 - 1) / (kT * 4), sms * 8u), kT, 0, st>>>(tris, sph, nt, n, cx, cy, cz,
+                                                                                       box);
+  k_morton<<<tiles, kT, 0, st>>>(cx, cy, cz, n, box, mode, ka, hist, tiles, tile);
   uint32_t *kin = ka, *vin = va, *kout = kb, *vout = vb;
   for (int pass = 0; pass < 4; ++pass) {
     const uint32_t shift = 8u * (uint32_t)pass;
     const uint32_t* v = pass ? vin : nullptr;
-    k_rs_hist<<<tiles, kT, 0, st>>>(kin, n, shift, hist, tiles, tile);
+    if (pass) k_rs_hist<<<tiles, kT, 0, st>>>(kin, n, shift, hist, tiles, tile);
     k_rs_scan<<<kBins, kT, 0, st>>>(hist, tiles, totals);
     if (tile == kT * kItemsSmall)
       k_rs_scatter<kItemsSmall><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
@@ -566,10 +668,9 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
     std::swap(kin, kout);
     std::swap(vin, vout);
   }
-  if ((e = cudaMemsetAsync(num_open, 0, 4 + (size_t)n * 4, st)) != cudaSuccess) return e;
   k_tree<<<blocks, kLeaves, 0, st>>>(tris, sph, nt, n, mode, kin, vin, nodes, open, num_open);
   if (blocks > 1)
-    k_top<<<std::min<uint32_t>(blocks, (uint32_t)device_sm_count() * 16u), 128, 0, st>>>(n, kin, open, num_open, slots,
+    k_top<<<std::min<uint32_t>(blocks, sms * 16u), 128, 0, st>>>(n, kin, open, num_open, slots,
                                                                                          nodes);
   return cudaGetLastError();
 }
