@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   dev::StepEntry stack[STACK];
   using Stk = typename std::conditional<(RING > 0), dev::RingStack<(RING > 0 ? RING : 1), THREADS, dev::StepEntry>,
                                         dev::LocalStackT<dev::StepEntry>>::type;
+  constexpr bool kDrain = !ANY && RING == 16;  // see k_trace_step
   Stk stk;
   if constexpr (RING > 0) {
     __shared__ dev::StepEntry ring[RING * THREADS];
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   const int min_idle = refill < 1 ? 1 : (refill > 32 ? 32 : refill);
   for (;;) {
     const uint32_t idle = __ballot_sync(0xFFFFFFFFu, local == 0xFFFFFFFFu);
-    if (exhausted && idle == 0xFFFFFFFFu) break;
+    if (exhausted && (kDrain || idle == 0xFFFFFFFFu)) break;
     if (!exhausted && __popc(idle) >= min_idle) {
       // One binary search per refill, for the first ray handed out; the
       // warp's other new rays follow it in the queue, so each lane walks on
@@ -213,6 +214,14 @@ __global__ void __launch_bounds__(THREADS, MINB)
       __stcs(&jobs[job].hits[local], h);  // written once: evict-first
       local = 0xFFFFFFFFu;
     }
+  }
+  if constexpr (kDrain) {
+    auto write = [&](uint32_t j, uint32_t i, uint32_t best, float t, bool overflow) {
+      uint2 h = make_uint2(RT_NO_HIT, 0x7f800000u);
+      if (!overflow && best != dev::kNoBest) h = make_uint2(__ldg(&S.tri_ids[best & kSlotMask]), __float_as_uint(t));
+      __stcs(&jobs[j].hits[i], h);
+    };
+    dev::drain<STACK, THREADS, false>(S, s, local != 0xFFFFFFFFu, job, local, stk.ring, stack, stk.lo, write);
   }
 }
 

@@ -140,6 +140,10 @@ __global__ void __launch_bounds__(THREADS, MINB)
   dev::StepEntry stack[STACK];
   using Stk = typename std::conditional<(RING > 0), dev::RingStack<(RING > 0 ? RING : 1), THREADS, dev::StepEntry>,
                                         dev::LocalStackT<dev::StepEntry>>::type;
+  // Any hit keeps a lane per ray to its end: which hit is found first must not
+  // depend on the warp's other rays.  The counting kernels count the
+  // sequential traversal.
+  constexpr bool kDrain = !ANY && !STATS && RING == 16;
   Stk stk;
   if constexpr (RING > 0) {
     __shared__ dev::StepEntry ring[RING * THREADS];
@@ -170,7 +174,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   const bool rays_al32 = dev::aligned32(rays);
   for (;;) {
     const uint32_t idle = __ballot_sync(0xFFFFFFFFu, ray == 0xFFFFFFFFu);
-    if (exhausted && idle == 0xFFFFFFFFu) break;
+    if (exhausted && (kDrain || idle == 0xFFFFFFFFu)) break;
     if (!exhausted && __popc(idle) >= min_idle) {
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(counter, (uint32_t)__popc(idle));
@@ -235,6 +239,24 @@ __global__ void __launch_bounds__(THREADS, MINB)
       }
       ray = 0xFFFFFFFFu;
     }
+  }
+  if constexpr (kDrain) {
+    auto write = [&](uint32_t id, uint32_t, uint32_t best, float t, bool overflow) {
+      uint2 h = make_uint2(best, __float_as_uint(t));
+      if (RAW) {
+        if (overflow) h.x = kRawOverflow;
+        hits[id] = h;
+        return;
+      }
+      if (overflow || best == dev::kNoBest)
+        h = make_uint2(RT_NO_HIT, 0x7f800000u);
+      else if (best & kSphereBit)
+        h.x = (best & kSphereMask) | RT_HIT_SPHERE_BIT;
+      else
+        h.x = __ldg(&S.tri_ids[best & kSlotMask]);
+      __stcs(&hits[id], h);
+    };
+    dev::drain<STACK, THREADS, MT>(S, s, ray != 0xFFFFFFFFu, ray, 0u, stk.ring, stack, stk.lo, write);
   }
   if constexpr (STATS) {
     for (int o = 16; o > 0; o >>= 1) {

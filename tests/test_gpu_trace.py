@@ -622,3 +622,36 @@ def test_ray_and_hit_alignment(rt, orc, cuda):
             assert f(sc.handle, buf.data_ptr() + roff, n, hits.data_ptr() + hoff, 0, st) == 1  # RT_EINVAL
             assert b"aligned" in rt.lib().rt_last_error_string()
     assert (ref["prim"] != orc.NO_HIT).sum() > n // 10
+
+
+@pytest.mark.parametrize("scene", ["duplicates", "cluster", "leaf4", "spheres", "one"])
+@pytest.mark.parametrize("n", [1, 31, 33, 5_001, 200_003])
+def test_shared_drain_is_sequential(rt, cuda, scene, n):
+    """A warp's last rays are finished by all of its lanes: bit for bit the hits of the launch shape whose lanes
+    each finish their own (stack in local memory), also where every hit is an exact tie between duplicates,
+    where stacks are deep, with leaves of several triangles and with spheres."""
+    kw = {}
+    if scene == "cluster":
+        tris, rays = _dense_cluster(rt, 3_000, 5), _rays_at_origin(rt, min(n, 20_001), 6)
+    else:
+        tris = rt.gen_soup(31, 0, 4_000, 1.0, 0.02)
+        rays = rt.gen_rays(31, 0, n, 1.0, 1e-4, float("inf"))
+        rays["tmax"][::3] = np.float32(0.2)
+    if scene == "duplicates":
+        tris = np.tile(tris[:800], 5)[np.random.default_rng(31).permutation(4_000)]
+    elif scene == "leaf4":
+        kw["leaf_size"] = 4
+    elif scene == "spheres":
+        sph = np.zeros(300, rt.SPHERE_DTYPE)
+        sph["center"][:, :3] = np.random.default_rng(32).random((300, 3)).astype(np.float32)
+        sph["radius"] = np.float32(0.03)
+        kw["spheres"] = sph
+    elif scene == "one":
+        tris = tris[:1]
+    with rt.Scene(tris, **kw) as sc:
+        got = dev_trace(rt, cuda, sc, rays)
+        got_sorted = dev_trace(rt, cuda, sc, rays, sort=True)
+        sc.set_tuning(rt.TraceTuning(14, 5, 0, 0, 0.0))
+        want = dev_trace(rt, cuda, sc, rays)
+    assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
+    assert np.array_equal(got_sorted.view(np.uint64), want.view(np.uint64))
