@@ -510,9 +510,7 @@ rt_status rt_trace(rt_scene* scene, const RtRay* d_rays, uint32_t n, RtHit* d_hi
   if (s != RT_OK) return s;
   uint32_t* order = nullptr;
   if ((s = maybe_reorder(w, scene->d, d_rays, n, flags, st, &order)) != RT_OK) return s;
-  cudaError_t e = cudaMemsetAsync(w->counters, 0, 2 * sizeof(uint32_t), st);
-  if (e != cudaSuccess) return cuda_fail(e, "rt_trace: memset");
-  e = launch_trace_tuned(scene->d, d_rays, n, d_hits, flags, w->counters, stream,
+  cudaError_t e = launch_trace_tuned(scene->d, d_rays, n, d_hits, flags, w->counters, stream,
                          (flags & RT_TRACE_MT) ? default_tuning() : scene->tune, nullptr, order);
   if (e != cudaSuccess) return cuda_fail(e, "rt_trace: launch");
   return RT_OK;
@@ -573,7 +571,6 @@ rt_status rt_trace_autotune(rt_scene* scene, const RtRay* d_rays, uint32_t n, Rt
     cudaError_t r = cudaSuccess;
     for (uint32_t k = 0; k <= repeats && r == cudaSuccess; ++k) {
       if (k == 1) r = cudaEventRecord(a, st);
-      if (r == cudaSuccess) r = cudaMemsetAsync(w->counters, 0, 2 * sizeof(uint32_t), st);
       if (r == cudaSuccess) r = launch_trace_tuned(scene->d, d_rays, n, d_hits, flags, w->counters, stream, t, nullptr, order);
     }
     if (r == cudaSuccess) r = cudaEventRecord(b, st);
@@ -790,8 +787,6 @@ rt_status rt_trace_host(rt_scene* scene, const RtRay* h_rays, uint32_t n, RtHit*
       uint32_t* order = nullptr;
       rt_status rs = maybe_reorder(w, scene->d, drays[b], cnt, flags, tst[b], &order, b * slot);
       if (rs != RT_OK) return rs;
-      if ((e = cudaMemsetAsync(counters[b], 0, 2 * sizeof(uint32_t), tst[b])) != cudaSuccess)
-        return cuda_fail(e, "memset");
       RtHit* out = direct ? direct + off : dhits[b];
       if ((e = launch_trace_tuned(scene->d, drays[b], cnt, out, flags, counters[b], tst[b],
                                   (flags & RT_TRACE_MT) ? default_tuning() : scene->tune, nullptr, order)) != cudaSuccess)

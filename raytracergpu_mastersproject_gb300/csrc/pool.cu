@@ -97,7 +97,8 @@ struct PoolTiledNodes {
 // (see k_trace_step).
 template <bool ANY, int STACK, int THREADS, int MINB, int RING, int TILE = 0, int VISITS = 1>
 __global__ void __launch_bounds__(THREADS, MINB)
-    k_pool_step(DeviceScene S, const DJob* __restrict__ table, uint32_t* __restrict__ counter, int refill) {
+    k_pool_step(DeviceScene S, const DJob* __restrict__ table, uint32_t* __restrict__ counter, int refill,
+                uint32_t spread) {
   dev::StepEntry stack[STACK];
   using Stk = typename std::conditional<(RING > 0), dev::RingStack<(RING > 0 ? RING : 1), THREADS, dev::StepEntry>,
                                         dev::LocalStackT<dev::StepEntry>>::type;
@@ -136,53 +137,61 @@ __global__ void __launch_bounds__(THREADS, MINB)
     fetch.count = 0u;
   }
   uint32_t job = 0, local = 0xFFFFFFFFu;
-  bool exhausted = total == 0;
   const int min_idle = refill < 1 ? 1 : (refill > 32 ? 32 : refill);
+  // Hands the queue's rays from `base` on to the lanes of `idle`.  One binary
+  // search per refill, for the first of them; the warp's other new rays follow
+  // it in the queue, so each lane walks on from that job (jobs hold thousands
+  // of rays: rarely a step, and never more than 8 before it searches for
+  // itself).
+  auto take = [&](uint32_t base, uint32_t idle) {
+    uint32_t first_job = 0;
+    if (lane == 0 && base < total) first_job = find_job(jobs, num_jobs, base);
+    first_job = __shfl_sync(0xFFFFFFFFu, first_job, 0);
+    const uint32_t g = base + (uint32_t)__popc(idle & lanemask_lt_p());
+    if ((idle >> lane & 1u) && g < total) {
+      job = first_job;
+      for (int k = 0; job + 1u < num_jobs && __ldg(&jobs[job + 1u].start) <= g; ++k) {
+        if (k == 8) {
+          job = find_job(jobs, num_jobs, g);
+          break;
+        }
+        ++job;
+      }
+      local = g - __ldg(&jobs[job].start);
+      const float4* rays = jobs[job].rays;
+      const uint32_t root = __ldg(&jobs[job].root);
+      float4 ro, rd;
+      dev::load_ray(rays, local, dev::aligned32(rays), ro, rd);
+      dev::trav_init_ray(s, ro, rd, root);
+      if constexpr (TILE > 0) {
+        fetch.tile = tile_base + 4u * TILE * job;
+        fetch.base = root;
+        fetch.count = tiled && root < kSentinel ? min((uint32_t)TILE, __ldg(&jobs[job].nodes)) : 0u;
+      }
+      stk.reset();
+      if (s.leaf != 0u) {
+        s.node = s.leaf;
+        s.leaf = 0u;
+      }
+    }
+  };
+  uint32_t queue = 0u;
+  bool exhausted = total == 0;
+  if constexpr (kDrain) {  // a warp's first rays are its own by position
+    const dev::Share own = dev::share_of<THREADS>(total, spread);
+    if (own.lanes) take(own.first, 0xFFFFFFFFu >> (32u - own.lanes));
+    queue = own.rest;
+    exhausted = own.rest >= total;
+  }
   for (;;) {
     const uint32_t idle = __ballot_sync(0xFFFFFFFFu, local == 0xFFFFFFFFu);
     if (exhausted && (kDrain || idle == 0xFFFFFFFFu)) break;
     if (!exhausted && __popc(idle) >= min_idle) {
-      // One binary search per refill, for the first ray handed out; the
-      // warp's other new rays follow it in the queue, so each lane walks on
-      // from that job (jobs hold thousands of rays: rarely a step, and
-      // never more than 8 before it searches for itself).
-      uint32_t base = 0, first_job = 0;
-      if (lane == 0) {
-        base = atomicAdd(counter, (uint32_t)__popc(idle));
-        if (base < total) first_job = find_job(jobs, num_jobs, base);
-      }
+      uint32_t base = 0;
+      if (lane == 0) base = queue + atomicAdd(counter, (uint32_t)__popc(idle));
       base = __shfl_sync(0xFFFFFFFFu, base, 0);
-      first_job = __shfl_sync(0xFFFFFFFFu, first_job, 0);
       if (base + (uint32_t)__popc(idle) >= total) exhausted = true;
-      if (local == 0xFFFFFFFFu) {
-        const uint32_t g = base + (uint32_t)__popc(idle & lanemask_lt_p());
-        if (g < total) {
-          job = first_job;
-          for (int k = 0; job + 1u < num_jobs && __ldg(&jobs[job + 1u].start) <= g; ++k) {
-            if (k == 8) {
-              job = find_job(jobs, num_jobs, g);
-              break;
-            }
-            ++job;
-          }
-          local = g - __ldg(&jobs[job].start);
-          const float4* rays = jobs[job].rays;
-          const uint32_t root = __ldg(&jobs[job].root);
-          float4 ro, rd;
-          dev::load_ray(rays, local, dev::aligned32(rays), ro, rd);
-          dev::trav_init_ray(s, ro, rd, root);
-          if constexpr (TILE > 0) {
-            fetch.tile = tile_base + 4u * TILE * job;
-            fetch.base = root;
-            fetch.count = tiled && root < kSentinel ? min((uint32_t)TILE, __ldg(&jobs[job].nodes)) : 0u;
-          }
-          stk.reset();
-          if (s.leaf != 0u) {
-            s.node = s.leaf;
-            s.leaf = 0u;
-          }
-        }
-      }
+      take(base, idle);
     }
     if (local == 0xFFFFFFFFu) continue;
     bool done = false;
@@ -225,7 +234,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   }
 }
 
-using PoolKernel = void (*)(DeviceScene, const DJob*, uint32_t*, int);
+using PoolKernel = void (*)(DeviceScene, const DJob*, uint32_t*, int, uint32_t);
 
 struct PoolVariant {
   int threads, minb, ring;
@@ -523,7 +532,7 @@ rt_status capture(rt_pool* P, LaunchSlot& sl, uint32_t* counter, int variant, in
   if (e == cudaSuccess) e = cudaMemsetAsync(counter, 0, 8, cs);
   if (e == cudaSuccess) {
     const uint32_t blocks = (uint32_t)(device_sm_count() * bps);
-    k<<<blocks, threads, 0, cs>>>(arena_view(P), sl.dev, counter, refill);
+    k<<<blocks, threads, 0, cs>>>(arena_view(P), sl.dev, counter, refill, spread_warps());
     e = cudaGetLastError();
   }
   cudaGraph_t g = nullptr;

@@ -201,7 +201,7 @@ cudaError_t launch_trace_tuned(const DeviceScene& s, const RtRay* rays, uint32_t
 size_t reorder_scratch_bytes(uint32_t n);
 cudaError_t launch_reorder(const DeviceScene& s, const RtRay* rays, uint32_t n, void* scratch, uint32_t** order_out,
                            void* stream);
-// Kernels launch on the given stream; counter is a device uint32 zeroed by the caller.
+// Kernels launch on the given stream; counter is a device uint32 (cleared by the launch where it is used).
 cudaError_t launch_trace(const DeviceScene& s, const RtRay* rays, uint32_t n, RtHit* hits, uint32_t flags,
                          uint32_t* counter, void* stream, const uint32_t* order = nullptr);
 // Path-tracer queries (render.cu): hits[i] = (leaf-style ref of the closest
@@ -237,6 +237,7 @@ size_t render_scratch_bytes(uint64_t paths, uint32_t depth);
 cudaError_t launch_accum_clear(float* accum, uint32_t w, uint32_t h, void* stream);
 cudaError_t launch_resolve(const float* accum, uint32_t w, uint32_t h, uint32_t spp, float* out, void* stream);
 int device_sm_count();
+uint32_t spread_warps();  // see trace.cu
 // GPU LBVH build (gpu_build.cu)
 size_t device_build_scratch_bytes(uint32_t n);
 cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtSphere32* sph, uint32_t ns,

@@ -34,7 +34,7 @@ template <bool ANY, int STACK, int THREADS, int MINB, int W, bool STATS, bool MT
 __global__ void __launch_bounds__(THREADS, MINB)
     k_trace(DeviceScene S, const float4* __restrict__ rays, uint32_t n, uint2* __restrict__ hits,
             uint32_t* __restrict__ counter, int refill, unsigned long long* __restrict__ stats,
-            const uint32_t* __restrict__ order) {
+            const uint32_t* __restrict__ order, uint32_t) {
   using StackT = typename std::conditional<W == 2, uint32_t, uint2>::type;
   StackT stack[STACK];
   dev::Trav s;
@@ -136,7 +136,7 @@ template <bool ANY, int STACK, int THREADS, int MINB, bool STATS, bool RAW = fal
 __global__ void __launch_bounds__(THREADS, MINB)
     k_trace_step(DeviceScene S, const float4* __restrict__ rays, uint32_t n, uint2* __restrict__ hits,
                  uint32_t* __restrict__ counter, int refill, unsigned long long* __restrict__ stats,
-            const uint32_t* __restrict__ order) {
+                 const uint32_t* __restrict__ order, uint32_t spread) {
   dev::StepEntry stack[STACK];
   using Stk = typename std::conditional<(RING > 0), dev::RingStack<(RING > 0 ? RING : 1), THREADS, dev::StepEntry>,
                                         dev::LocalStackT<dev::StepEntry>>::type;
@@ -168,32 +168,43 @@ __global__ void __launch_bounds__(THREADS, MINB)
   const uint32_t lane = threadIdx.x & 31u;
   if (RAW && n == 0xFFFFFFFFu) n = *reinterpret_cast<volatile uint32_t*>(counter + 2);
   uint32_t ray = 0xFFFFFFFFu;
-  bool exhausted = false;
   unsigned long long vis = 0, tests = 0;
   const int min_idle = refill < 1 ? 1 : (refill > 32 ? 32 : refill);
   const bool rays_al32 = dev::aligned32(rays);
+  auto start = [&](uint32_t id) {
+    if (id < n && !dev::chk(S.check, order && __ldg(&order[id]) >= n, dev::kChkRay, order ? __ldg(&order[id]) : id)) {
+      ray = order ? __ldg(&order[id]) : id;
+      float4 ro, rd;
+      dev::load_ray(rays, ray, rays_al32, ro, rd);
+      dev::trav_init_ray(s, ro, rd, S.root);
+      stk.reset();
+      if (s.leaf != 0u) {  // the whole tree is one leaf
+        s.node = s.leaf;
+        s.leaf = 0u;
+      }
+    }
+  };
+  // The queue hands out all rays of an any-hit or counting launch.  In the
+  // others a warp's first rays are its own by position, and the queue hands out
+  // the rest (none when the grid has a lane for every ray: then it need not be
+  // cleared either).
+  uint32_t queue = 0u;
+  bool exhausted = false;
+  if constexpr (kDrain) {
+    const dev::Share own = dev::share_of<THREADS>(n, spread);
+    if (lane < own.lanes) start(own.first + lane);
+    queue = own.rest;
+    exhausted = own.rest >= n;
+  }
   for (;;) {
     const uint32_t idle = __ballot_sync(0xFFFFFFFFu, ray == 0xFFFFFFFFu);
     if (exhausted && (kDrain || idle == 0xFFFFFFFFu)) break;
     if (!exhausted && __popc(idle) >= min_idle) {
       uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(counter, (uint32_t)__popc(idle));
+      if (lane == 0) base = queue + atomicAdd(counter, (uint32_t)__popc(idle));
       base = __shfl_sync(0xFFFFFFFFu, base, 0);
       if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
-      if (ray == 0xFFFFFFFFu) {
-        const uint32_t id = base + (uint32_t)__popc(idle & lanemask_lt());
-        if (id < n && !dev::chk(S.check, order && __ldg(&order[id]) >= n, dev::kChkRay, order ? __ldg(&order[id]) : id)) {
-          ray = order ? __ldg(&order[id]) : id;
-          float4 ro, rd;
-          dev::load_ray(rays, ray, rays_al32, ro, rd);
-          dev::trav_init_ray(s, ro, rd, S.root);
-          stk.reset();
-          if (s.leaf != 0u) {  // the whole tree is one leaf
-            s.node = s.leaf;
-            s.leaf = 0u;
-          }
-        }
-      }
+      if (ray == 0xFFFFFFFFu) start(base + (uint32_t)__popc(idle & lanemask_lt()));
     }
     if (ray == 0xFFFFFFFFu) continue;
     bool done = false;
@@ -271,13 +282,14 @@ __global__ void __launch_bounds__(THREADS, MINB)
 }
 
 using TraceKernel = void (*)(DeviceScene, const float4*, uint32_t, uint2*, uint32_t*, int, unsigned long long*,
-                             const uint32_t*);
+                             const uint32_t*, uint32_t);
 
 // Stack capacities: binary trees 64 or 128 refs (depth + sentinel); 4-wide
 // trees 64 or 192 entries (worst-case pushes along a path; (ref, t_near) in
 // the while-while loop, the ref alone in the step loop).
 struct Variant {
   int threads, minb;
+  bool drain;  // closest hit on 4-wide trees ends in the shared drain (step loop with the ring)
   TraceKernel k[2][2][2][2];  // [stats][wide][any][big stack]
   int blocks_per_sm[2][2][2][2];
 };
@@ -308,6 +320,7 @@ Variant make_variant() {
   Variant v;
   v.threads = T;
   v.minb = M;
+  v.drain = STEP && RING == 16;
   if constexpr (STEP) {
     fill_step_variant<T, M, false, RING, VISITS>(v);
     fill_step_variant<T, M, true, RING, VISITS>(v);
@@ -446,16 +459,33 @@ cudaError_t launch_trace_tuned(const DeviceScene& S, const RtRay* rays, uint32_t
   }
   int bps = 0;
   if (cudaError_t e = cached_blocks_per_sm(slot, k, threads, &bps); e != cudaSuccess) return e;
-  const uint32_t warps_per_block = (uint32_t)threads / 32u;
-  const uint32_t warps_needed = (n + 31u) / 32u;
+  // these kernels hand out their first rays by position (see k_trace_step)
+  const bool drain = wide && !any && !stats && (mt || v.drain);
   uint64_t blocks = (uint64_t)device_sm_count() * (uint64_t)bps * (uint64_t)std::max(1, tune.grid_scale) / 100u;
-  const uint64_t needed = (warps_needed + warps_per_block - 1) / warps_per_block;
+  uint64_t needed = ((uint64_t)n + threads - 1) / threads;
+  if (drain) {  // few rays: a ray per warp at least, over up to `spread` warps
+    const uint64_t wpb = (uint64_t)threads / 32u;
+    needed = std::max(needed, std::min<uint64_t>(n, spread_warps()) / wpb + 1u);
+  }
   if (blocks > needed) blocks = needed;
   if (blocks == 0) blocks = 1;
+  // a grid of theirs with a lane for every ray never looks at the queue
+  if (!drain || n > blocks * (uint64_t)threads) {
+    const cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return e;
+  }
   k<<<(uint32_t)blocks, threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      S, reinterpret_cast<const float4*>(rays), n, reinterpret_cast<uint2*>(hits), counter, tune.refill, stats, order);
+      S, reinterpret_cast<const float4*>(rays), n, reinterpret_cast<uint2*>(hits), counter, tune.refill, stats, order,
+      spread_warps());
   return cudaGetLastError();
 }
+
+// Warps over which a closest-hit step-loop launch spreads fewer rays than they
+// have lanes: eight per SM, two per scheduler, which still leaves every warp's
+// chain of fetches nearly to itself.  17 rays on 20,482 triangles take 12.3 us
+// so and 14.9 in one warp; a 317x179 preview's four bounce levels 124 against
+// 157 us (4 and 16 warps per SM: 124 and 121).
+uint32_t spread_warps() { return (uint32_t)device_sm_count() * 8u; }
 
 int device_sm_count() {
   static int cached = -1;
@@ -496,12 +526,14 @@ cudaError_t launch_trace_raw(const DeviceScene& S, const float4* rays, uint32_t 
   int per_sm = 0;
   if (cudaError_t e = cached_blocks_per_sm(&bps[k], kern, T, &per_sm); e != cudaSuccess) return e;
   uint64_t blocks = (uint64_t)device_sm_count() * (uint64_t)per_sm;
-  if (n != 0xFFFFFFFFu) blocks = std::min<uint64_t>(blocks, ((uint64_t)n + T - 1) / T);
+  if (n != 0xFFFFFFFFu)
+    blocks = std::min<uint64_t>(blocks, std::max<uint64_t>(((uint64_t)n + T - 1) / T,
+                                                           std::min<uint64_t>(n, spread_warps()) / (T / 32) + 1u));
   if (blocks == 0) blocks = 1;
   // The path tracer's bounce rays are short: refilling at 8 idle lanes beats
   // 4 there (config 2: 3.49 against 3.53 ms per frame).
   static const int refill = env_int("RT_TRACE_RAW_REFILL", 8);
-  kern<<<(uint32_t)blocks, T, 0, st>>>(S, rays, n, hits, counter, refill, stats, nullptr);
+  kern<<<(uint32_t)blocks, T, 0, st>>>(S, rays, n, hits, counter, refill, stats, nullptr, spread_warps());
   return cudaGetLastError();
 }
 
@@ -544,14 +576,6 @@ extern "C" rt_status rt_trace_noalloc(rt_scene* scene, const RtRay* d_rays, uint
       return RT_ECUDA;
     }
     scratch = static_cast<uint32_t*>(p);
-  }
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // The array keeps the previous call's contents: the queue counter must
-  // start at zero.
-  e = cudaMemsetAsync(scratch, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) {
-    set_error(std::string("rt_trace_noalloc: memset: ") + cudaGetErrorString(e));
-    return RT_ECUDA;
   }
   e = launch_trace(*scene_device(scene), d_rays, n, d_hits, flags, scratch, stream);
   if (e != cudaSuccess) {

@@ -149,6 +149,24 @@ __device__ __forceinline__ bool sphere_test(const void* spheres, uint32_t idx, f
   return true;
 }
 
+// ------------------------------------------------------- ray hand-out ----
+// The rays of a step-loop launch that a warp takes by position, before the
+// queue: a ray per lane, or fewer where n rays would otherwise leave some of
+// `spread` warps without one.
+struct Share {
+  uint32_t lanes;        // lanes that carry rays
+  uint32_t first, rest;  // the warp's first ray; the queue's first ray
+};
+template <int THREADS>
+__device__ __forceinline__ Share share_of(uint32_t n, uint32_t spread) {
+  Share s;
+  const uint32_t warps = gridDim.x * (THREADS / 32), over = min(warps, spread);
+  s.lanes = n >= 32u * over ? 32u : (n + over - 1u) / over;  // below 32 there is a lane for every ray
+  s.first = (blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5)) * s.lanes;
+  s.rest = warps * s.lanes;
+  return s;
+}
+
 // ---------------------------------------------------------- traversal ----
 // One ray's traversal state; kept in registers across warp refills.
 #ifndef RT_DEVICE_CHECKS
@@ -741,7 +759,9 @@ __device__ __forceinline__ void drain(const DeviceScene& S, Trav& s, bool busy, 
     if (busy) {
       const float t = __uint_as_float(W[9 * T + slot]);
       if (t < s.tclose) trav_set_close(s, t);
-      overflow = !drain_step<STACK, MT>(S, s, stk);
+      // a ray that never enters the tree (an empty scene, a component that is
+      // not finite) starts at the sentinel
+      if (s.node != kSentinel) overflow = !drain_step<STACK, MT>(S, s, stk);
     }
     __syncwarp();
     for (uint32_t found = __ballot_sync(0xFFFFFFFFu, busy && s.best != kNoBest); found != 0u; found &= found - 1u) {
