@@ -138,13 +138,13 @@ static rt_status ensure_helpers(Workspace* w) {
 
 static size_t sort_slot_bytes(uint32_t n) { return (reorder_scratch_bytes(n) + 255) & ~(size_t)255; }
 
-// Reorders the batch when RT_TRACE_SORT is set; *order = nullptr otherwise.
+// Reorders the batch when RT_TRACE_SORT is set and it pays; *order = nullptr otherwise.
 // The scratch starts `offset` bytes into the workspace's sort buffer, so that
 // batches in flight on two streams use disjoint regions.
 static rt_status maybe_reorder(Workspace* w, const DeviceScene& d, const RtRay* rays, uint32_t n, uint32_t flags,
                                cudaStream_t st, uint32_t** order, size_t offset = 0) {
   *order = nullptr;
-  if (!(flags & RT_TRACE_SORT) || d.root == kSentinel) return RT_OK;
+  if (!(flags & RT_TRACE_SORT) || d.root == kSentinel || !reorder_pays(d, n)) return RT_OK;
   rt_status s = ensure_sort_scratch(w, offset + reorder_scratch_bytes(n));
   if (s != RT_OK) return s;
   cudaError_t e = launch_reorder(d, rays, n, static_cast<char*>(w->sort) + offset, order, st);
@@ -744,7 +744,8 @@ rt_status rt_trace_host(rt_scene* scene, const RtRay* h_rays, uint32_t n, RtHit*
     w->stage_bytes = need;
   }
   const size_t slot = sort_slot_bytes(chunk);
-  if ((flags & RT_TRACE_SORT) && (s = ensure_sort_scratch(w, 2 * slot)) != RT_OK) return s;
+  if ((flags & RT_TRACE_SORT) && reorder_pays(scene->d, chunk) && (s = ensure_sort_scratch(w, 2 * slot)) != RT_OK)
+    return s;
   if ((s = ensure_helpers(w)) != RT_OK) return s;
   char* base = static_cast<char*>(w->stage);
   RtRay* drays[2] = {reinterpret_cast<RtRay*>(base), reinterpret_cast<RtRay*>(base + per)};

@@ -196,8 +196,10 @@ bool tuning_supported(const TraceTuning& t, uint32_t width, uint32_t stack_need,
 cudaError_t launch_trace_tuned(const DeviceScene& s, const RtRay* rays, uint32_t n, RtHit* hits, uint32_t flags,
                                uint32_t* counter, void* stream, const TraceTuning& tune,
                                unsigned long long* stats, const uint32_t* order);
-// Coherence reordering (reorder.cu): bytes of scratch for n rays, and the
-// launch that leaves the ray order (a permutation of 0..n-1) in *order_out.
+// Coherence reordering (reorder.cu): whether it pays for n rays, bytes of
+// scratch for them, and the launch that leaves the ray order (a permutation of
+// 0..n-1) in *order_out.
+bool reorder_pays(const DeviceScene& s, uint32_t n);
 size_t reorder_scratch_bytes(uint32_t n);
 cudaError_t launch_reorder(const DeviceScene& s, const RtRay* rays, uint32_t n, void* scratch, uint32_t** order_out,
                            void* stream);

@@ -655,3 +655,14 @@ def test_shared_drain_is_sequential(rt, cuda, scene, n):
         want = dev_trace(rt, cuda, sc, rays)
     assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
     assert np.array_equal(got_sorted.view(np.uint64), want.view(np.uint64))
+
+
+@pytest.mark.parametrize("n", [1_572_863, 1_572_864, 2_000_001])
+def test_sorted_order_same_hits(rt, cuda, n):
+    """On a tree beyond L2 a sorted batch is reordered from 1,572,864 rays on; hits do not change."""
+    tris = rt.gen_soup(33, 0, 1_500_000, 1.0, 0.002)
+    rays = rt.gen_rays(33, 0, n, 1.0, 1e-4, float("inf"))
+    with rt.Scene(tris) as sc:
+        want = dev_trace(rt, cuda, sc, rays).view(np.uint64)
+        assert np.array_equal(dev_trace(rt, cuda, sc, rays, sort=True).view(np.uint64), want)
+        assert np.array_equal(sc.trace_host(rays, sort=True).view(np.uint64), want)
