@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   dev::StepEntry stack[STACK];
   using Stk = typename std::conditional<(RING > 0), dev::RingStack<(RING > 0 ? RING : 1), THREADS, dev::StepEntry>,
                                         dev::LocalStackT<dev::StepEntry>>::type;
-  constexpr bool kDrain = !ANY && RING == 16;  // see k_trace_step
+  constexpr bool kDrain = RING == 16;  // see k_trace_step
   Stk stk;
   if constexpr (RING > 0) {
     __shared__ dev::StepEntry ring[RING * THREADS];
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       if (!overflow && best != dev::kNoBest) h = make_uint2(__ldg(&S.tri_ids[best & kSlotMask]), __float_as_uint(t));
       __stcs(&jobs[j].hits[i], h);
     };
-    dev::drain<STACK, THREADS, false>(S, s, local != 0xFFFFFFFFu, job, local, stk.ring, stack, stk.lo, write);
+    dev::drain<ANY, STACK, THREADS, false>(S, s, local != 0xFFFFFFFFu, job, local, stk.ring, stack, stk.lo, write);
   }
 }
 

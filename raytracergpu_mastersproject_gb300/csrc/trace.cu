@@ -140,10 +140,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
   dev::StepEntry stack[STACK];
   using Stk = typename std::conditional<(RING > 0), dev::RingStack<(RING > 0 ? RING : 1), THREADS, dev::StepEntry>,
                                         dev::LocalStackT<dev::StepEntry>>::type;
-  // Any hit keeps a lane per ray to its end: which hit is found first must not
-  // depend on the warp's other rays.  The counting kernels count the
-  // sequential traversal.
-  constexpr bool kDrain = !ANY && !STATS && RING == 16;
+  // The counting kernels count the sequential traversal.
+  constexpr bool kDrain = !STATS && RING == 16;
   Stk stk;
   if constexpr (RING > 0) {
     __shared__ dev::StepEntry ring[RING * THREADS];
@@ -184,10 +182,9 @@ __global__ void __launch_bounds__(THREADS, MINB)
       }
     }
   };
-  // The queue hands out all rays of an any-hit or counting launch.  In the
-  // others a warp's first rays are its own by position, and the queue hands out
-  // the rest (none when the grid has a lane for every ray: then it need not be
-  // cleared either).
+  // Where a launch ends in the shared drain, a warp's first rays are its own by
+  // position, and the queue hands out the rest (none when the grid has a lane
+  // for every ray: then it need not be cleared either).
   uint32_t queue = 0u;
   bool exhausted = false;
   if constexpr (kDrain) {
@@ -267,7 +264,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
         h.x = __ldg(&S.tri_ids[best & kSlotMask]);
       __stcs(&hits[id], h);
     };
-    dev::drain<STACK, THREADS, MT>(S, s, ray != 0xFFFFFFFFu, ray, 0u, stk.ring, stack, stk.lo, write);
+    dev::drain<ANY, STACK, THREADS, MT>(S, s, ray != 0xFFFFFFFFu, ray, 0u, stk.ring, stack, stk.lo, write);
   }
   if constexpr (STATS) {
     for (int o = 16; o > 0; o >>= 1) {
@@ -289,7 +286,7 @@ using TraceKernel = void (*)(DeviceScene, const float4*, uint32_t, uint2*, uint3
 // the while-while loop, the ref alone in the step loop).
 struct Variant {
   int threads, minb;
-  bool drain;  // closest hit on 4-wide trees ends in the shared drain (step loop with the ring)
+  bool drain;  // 4-wide trees end in the shared drain (step loop with the ring)
   TraceKernel k[2][2][2][2];  // [stats][wide][any][big stack]
   int blocks_per_sm[2][2][2][2];
 };
@@ -460,7 +457,7 @@ cudaError_t launch_trace_tuned(const DeviceScene& S, const RtRay* rays, uint32_t
   int bps = 0;
   if (cudaError_t e = cached_blocks_per_sm(slot, k, threads, &bps); e != cudaSuccess) return e;
   // these kernels hand out their first rays by position (see k_trace_step)
-  const bool drain = wide && !any && !stats && (mt || v.drain);
+  const bool drain = wide && !stats && (mt || v.drain);
   uint64_t blocks = (uint64_t)device_sm_count() * (uint64_t)bps * (uint64_t)std::max(1, tune.grid_scale) / 100u;
   uint64_t needed = ((uint64_t)n + threads - 1) / threads;
   if (drain) {  // few rays: a ray per warp at least, over up to `spread` warps

@@ -606,10 +606,12 @@ __device__ __forceinline__ bool visit_wide_stk(const DeviceScene& S, Trav& s, St
 // end's bookkeeping).  Spreading a small launch's rays thinly over more warps
 // instead made it slower (304 -> 376): twice the warps contend for issue.
 //
-// The result is the sequential one: the minimum t over the same candidates, and
-// among equal t the candidate that is last in the ray's visiting order, which
-// the workers' ranks keep (a taken subtree comes after all that its giver
-// keeps).
+// The result is the sequential one, whichever lanes work on a ray: the minimum t
+// over the same candidates, and among equal t the candidate that is last in the
+// ray's visiting order, which the workers' ranks keep (a taken subtree comes
+// after all that its giver keeps).  Any hit: the hit of the lowest rank; a worker
+// of a higher rank stops, those of lower ranks go on, and nothing is culled, so
+// it is the first hit in the ray's order again.
 //
 // Each lane's 16 ring words are laid out anew: words 0-7 a ring of its stack's
 // top, 8 its rank, and, for the ray that started in the lane, 9-11 the best hit
@@ -649,6 +651,10 @@ struct DrainStack {
 // number of halvings in bits 0-4.  A giver keeps the lower half of its
 // interval, the taker gets the upper one.
 constexpr uint32_t kMaxHalvings = 26;
+// Idle lanes from which work changes hands: pairing costs about as many
+// instructions as a node visit (100,003 rays 182 us at 1, 177 at 8; a frame
+// 2,898 and 2,874).
+constexpr int kMinIdleDrain = 8;
 
 // One step of one lane: an inner node or one primitive.  A node and a triangle
 // record are both 64 bytes, so one pair of loads serves the lanes of either
@@ -690,7 +696,7 @@ __device__ __forceinline__ bool drain_step(const DeviceScene& S, Trav& s, Stk& s
 
 // `ring`: the lane's column of the block's 16 x T ring (entries [lo, s.sp) in
 // the main loop's layout); `write(id0, id1, ref, t, overflow)` stores a result.
-template <int STACK, int T, bool MT, class Write>
+template <bool ANY, int STACK, int T, bool MT, class Write>
 __device__ __forceinline__ void drain(const DeviceScene& S, Trav& s, bool busy, uint32_t id0, uint32_t id1,
                                       uint32_t* ring, uint32_t* spill, int lo, const Write& write) {
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
@@ -704,7 +710,7 @@ __device__ __forceinline__ void drain(const DeviceScene& S, Trav& s, bool busy, 
   ring[8 * T] = 0u;
   ring[9 * T] = s.best != kNoBest && busy ? fbits(s.tclose) : 0x7f800000u;
   ring[10 * T] = busy ? s.best : kNoBest;
-  ring[11 * T] = 0u;
+  ring[11 * T] = ANY ? 0xFFFFFFFFu : 0u;
   ring[12 * T] = busy ? 1u : 0u;
   ring[13 * T] = id0;
   ring[14 * T] = id1;
@@ -715,7 +721,7 @@ __device__ __forceinline__ void drain(const DeviceScene& S, Trav& s, bool busy, 
     if (idle == 0xFFFFFFFFu) break;
     const uint32_t givers =
         __ballot_sync(0xFFFFFFFFu, busy && s.sp > stk.bot && (ring[8 * T] & 31u) < kMaxHalvings);
-    if (idle != 0u && givers != 0u) {
+    if (__popc(idle) >= kMinIdleDrain && givers != 0u) {
       const int pairs = min(__popc(idle), __popc(givers));
       const int gi = __popc(givers & below), ti = __popc(idle & below);
       uint32_t entry = 0u, rank = 0u;
@@ -757,8 +763,12 @@ __device__ __forceinline__ void drain(const DeviceScene& S, Trav& s, bool busy, 
     }
     bool overflow = false;
     if (busy) {
-      const float t = __uint_as_float(W[9 * T + slot]);
-      if (t < s.tclose) trav_set_close(s, t);
+      if (ANY) {
+        if ((ring[8 * T] >> 5) > W[11 * T + slot]) s.node = kSentinel;  // an earlier hit is known
+      } else {
+        const float t = __uint_as_float(W[9 * T + slot]);
+        if (t < s.tclose) trav_set_close(s, t);
+      }
       // a ray that never enters the tree (an empty scene, a component that is
       // not finite) starts at the sentinel
       if (s.node != kSentinel) overflow = !drain_step<STACK, MT>(S, s, stk);
@@ -767,13 +777,14 @@ __device__ __forceinline__ void drain(const DeviceScene& S, Trav& s, bool busy, 
     for (uint32_t found = __ballot_sync(0xFFFFFFFFu, busy && s.best != kNoBest); found != 0u; found &= found - 1u) {
       if (lane == (uint32_t)__ffs(found) - 1u) {
         const float t = __uint_as_float(W[9 * T + slot]);
-        const uint32_t r = ring[8 * T] >> 5;
-        if (s.tclose < t || (s.tclose == t && r >= W[11 * T + slot])) {
+        const uint32_t r = ring[8 * T] >> 5, rt = W[11 * T + slot];
+        if (ANY ? r < rt : s.tclose < t || (s.tclose == t && r >= rt)) {
           W[9 * T + slot] = fbits(s.tclose);
           W[10 * T + slot] = s.best;
           W[11 * T + slot] = r;
         }
         s.best = kNoBest;
+        if (ANY) s.node = kSentinel;  // this worker's first hit
       }
       __syncwarp();
     }

@@ -649,12 +649,11 @@ def test_shared_drain_is_sequential(rt, cuda, scene, n):
     elif scene == "one":
         tris = tris[:1]
     with rt.Scene(tris, **kw) as sc:
-        got = dev_trace(rt, cuda, sc, rays)
-        got_sorted = dev_trace(rt, cuda, sc, rays, sort=True)
+        got = [dev_trace(rt, cuda, sc, rays, any_hit=a) for a in (False, True)]
         sc.set_tuning(rt.TraceTuning(14, 5, 0, 0, 0.0))
-        want = dev_trace(rt, cuda, sc, rays)
-    assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
-    assert np.array_equal(got_sorted.view(np.uint64), want.view(np.uint64))
+        want = [dev_trace(rt, cuda, sc, rays, any_hit=a) for a in (False, True)]
+    for g, w in zip(got, want):
+        assert np.array_equal(g.view(np.uint64), w.view(np.uint64))
 
 
 @pytest.mark.parametrize("n", [1_572_863, 1_572_864, 2_000_001])
