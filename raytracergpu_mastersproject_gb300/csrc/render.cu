@@ -401,11 +401,12 @@ __global__ void __launch_bounds__(THREADS, MINB)
 // p / ns: a pixel's samples start from the same hit point, and kept adjacent
 // they keep their next rays in the same warps.  The starting RNG states are
 // stored sample-major (rng0[k * npix + q]) so that k_wave_seed's stores are
-// coalesced.  Scratch per path: state (color.xyz, rng | gatt.xyz, -) 32 B,
-// the starting RNG state 4 B, two ray buffers 2 x 32 B, two path lists
-// 2 x 4 B, hits 8 B.
+// coalesced.  Scratch per path: the colour so far and RNG state 16 B, the
+// throughput 16 B (of continuing paths alone), the starting RNG state 4 B, two
+// ray buffers 2 x 32 B, two path lists 2 x 4 B, hits 8 B.
 struct WaveBufs {
-  float4* state;  // 2 float4 per path
+  float4* color;  // color.xyz, rng
+  float4* gatt;   // gatt.xyz, -
   uint32_t* rng0;
   float4* rays[2];
   uint32_t* list[2];
@@ -450,10 +451,19 @@ __global__ void k_wave_seed(Cam cam, uint32_t random_state, float4* __restrict__
 // rays[p] or, when the pixel's first hit is shared, rays[p / ns]; colour 0,
 // throughput 1, RNG from rng0); later levels take the count from the level's
 // counter block and path ids from `list`.
+//
+// Bound by the latency of its chain of loads (path -> hit -> triangle ->
+// material): 10 blocks of 128 threads per SM at 48 registers hide more of it than
+// 4 of 256 at 53 (and spill nothing; 12 blocks do).  With the throughput stored
+// for continuing paths alone and the colour where it changed, level 0 of half a
+// 1280x720 frame of 16 samples takes 92-146 us instead of 109-164, the frame
+// 2,770 instead of 2,864 us (2,809 with 4 blocks of 256).
+constexpr int kShadeThreads = 128, kShadeBlocks = 10;
 template <bool STATS>
-__global__ void k_wave_shade(DeviceScene S, uint32_t level, uint32_t depth, uint32_t n0, uint32_t npix, uint32_t ns,
+__global__ void __launch_bounds__(kShadeThreads, kShadeBlocks) k_wave_shade(DeviceScene S, uint32_t level, uint32_t depth, uint32_t n0, uint32_t npix, uint32_t ns,
                              uint32_t per_path, uint32_t mode, float bgx, float bgy, float bgz,
-                             float4* __restrict__ state, const uint32_t* __restrict__ rng0,
+                             float4* __restrict__ color_of, float4* __restrict__ gatt_of,
+                             const uint32_t* __restrict__ rng0,
                              const float4* __restrict__ rays, const uint32_t* __restrict__ list,
                              const uint2* __restrict__ hits, float4* __restrict__ next_rays,
                              uint32_t* __restrict__ next_list, uint32_t* __restrict__ cnt,
@@ -484,16 +494,19 @@ __global__ void k_wave_shade(DeviceScene S, uint32_t level, uint32_t depth, uint
       if (level == 0) {
         rng = rng0[(size_t)(p % ns) * npix + p / ns];
       } else {
-        const float4 a = state[2 * (size_t)p], g = state[2 * (size_t)p + 1];
+        const float4 a = color_of[p], g = gatt_of[p];
         color = mk(a.x, a.y, a.z);
         gatt = mk(g.x, g.y, g.z);
         rng = __float_as_uint(a.w);
       }
       co = mk(o.x, o.y, o.z);
       cd = mk(d.x, d.y, d.z);
+      const f3 before = color;
       more = bounce(S, s, co, cd, color, gatt, rng, extended, bg, status) && level + 1u < depth;
-      state[2 * (size_t)p] = make_float4(color.x, color.y, color.z, __uint_as_float(rng));
-      state[2 * (size_t)p + 1] = make_float4(gatt.x, gatt.y, gatt.z, 0.0f);
+      // an ended path needs its colour alone, and that only if it changed
+      if (more || level == 0 || color.x != before.x || color.y != before.y || color.z != before.z)
+        color_of[p] = make_float4(color.x, color.y, color.z, __uint_as_float(rng));
+      if (more) gatt_of[p] = make_float4(gatt.x, gatt.y, gatt.z, 0.0f);
     }
     // append the continuing paths: one atomicAdd per warp
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, more);
@@ -514,11 +527,12 @@ __global__ void k_wave_shade(DeviceScene S, uint32_t level, uint32_t depth, uint
 }
 
 __global__ void k_wave_accum(float4* __restrict__ accum, uint32_t pix0, uint32_t npix, uint32_t ns,
-                             const float4* __restrict__ state) {
+                             const float4* __restrict__ color_of) {
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < npix; q += gridDim.x * blockDim.x) {
     float4 px = accum[pix0 + q];
+#pragma unroll 8  // a 128-byte line of a thread's samples at once (41 -> 32 us)
     for (uint32_t k = 0; k < ns; ++k) {
-      const float4 c = state[2 * ((size_t)q * ns + k)];
+      const float4 c = color_of[(size_t)q * ns + k];
       px.x = c.x + px.x;
       px.y = c.y + px.y;
       px.z = c.z + px.z;
@@ -536,8 +550,10 @@ WaveBufs wave_bufs(void* scratch, uint64_t paths, uint32_t depth) {
   char* b = static_cast<char*>(scratch);
   WaveBufs w;
   size_t off = 0;
-  w.state = reinterpret_cast<float4*>(b + off);
-  off += up(paths * 32);
+  w.color = reinterpret_cast<float4*>(b + off);
+  off += up(paths * 16);
+  w.gatt = reinterpret_cast<float4*>(b + off);
+  off += up(paths * 16);
   w.rng0 = reinterpret_cast<uint32_t*>(b + off);
   off += up(paths * 4);
   w.rays[0] = reinterpret_cast<float4*>(b + off);
@@ -557,7 +573,7 @@ WaveBufs wave_bufs(void* scratch, uint64_t paths, uint32_t depth) {
 
 // Scratch of one stream's part for `paths` paths.
 size_t wave_part_bytes(uint64_t paths, uint32_t depth) {
-  const size_t b = (size_t)paths * kWaveBytesPerPath + 8 * 256 + 16 * ((size_t)depth + 1);
+  const size_t b = (size_t)paths * kWaveBytesPerPath + 9 * 256 + 16 * ((size_t)depth + 1);
   return (b + 255) & ~(size_t)255;  // the next stream's part starts 256-byte aligned
 }
 
@@ -622,13 +638,14 @@ cudaError_t launch_render_wave(const DeviceScene& S, const Cam& cam, uint32_t de
           if ((e2 = launch_trace_raw(S, r, l == 0 ? (per_path ? np : q) : 0xFFFFFFFFu, B.hits, B.cnt + 4u * l,
                                      trace_stats, cs)) != cudaSuccess)
             return e2;
-          const uint32_t gs = l == 0 ? std::min<uint32_t>(sms * 8, (np + 255) / 256) : sms * 8;
-          k_wave_shade<STATS><<<gs, 256, 0, cs>>>(S, l, depth, np, q, ns, per_path, mode, bg[0], bg[1], bg[2],
-                                                  B.state, B.rng0, r, B.list[l & 1u], B.hits,
-                                                  B.rays[(l + 1u) & 1u], B.list[(l + 1u) & 1u], B.cnt,
-                                                  counter + 1, stats);
+          uint32_t gs = sms * kShadeBlocks;
+          if (l == 0) gs = std::min<uint32_t>(gs, (np + kShadeThreads - 1) / kShadeThreads);
+          k_wave_shade<STATS><<<gs, kShadeThreads, 0, cs>>>(S, l, depth, np, q, ns, per_path, mode, bg[0], bg[1],
+                                                            bg[2], B.color, B.gatt, B.rng0, r, B.list[l & 1u], B.hits,
+                                                            B.rays[(l + 1u) & 1u], B.list[(l + 1u) & 1u], B.cnt,
+                                                            counter + 1, stats);
         }
-        k_wave_accum<<<gb, 256, 0, cs>>>(accum, pix0, q, ns, B.state);
+        k_wave_accum<<<gb, 256, 0, cs>>>(accum, pix0, q, ns, B.color);
         if ((e2 = cudaGetLastError()) != cudaSuccess) return e2;
       }
     }
