@@ -7,12 +7,14 @@
 //                    atomicMax on order-preserving integer images of floats
 //   k_morton         the box's padding (:105-109), 30-bit codes
 //                    (GenerateMortonCodesOfPrimitives.comp:52-93)
+//   k_front          all of the above and the sort in one cluster, small builds
 //   radix sort       stable LSD sort of (code, index), 4 passes of 8 bits like
 //                    RadixSortSimple.comp:8-13: per-tile histograms, a scan, and
 //                    a scatter whose ranks keep input order (warp multi-split)
 //   k_tree           padded leaf boxes (ConstructHLBVH.comp:117-169), internal
 //                    nodes (:72-209) and box unions, the second arriving child
 //                    continuing upward (ConstructAABBsOfInternalNodes.comp:38-64)
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -343,6 +345,163 @@ __global__ void __launch_bounds__(kT, 4) k_rs_scatter(const uint32_t* __restrict
   }
 }
 
+// ---- small builds: centroids, codes and sort in one cluster ----
+// Below kFrontMax primitives the twelve launches above are bound by their gaps
+// and by a few blocks' latency.  Here eight blocks of one cluster hold all keys
+// in their shared memory: block r sorted positions [r M, (r + 1) M).  The box is
+// reduced and each pass's digit counts are exchanged through distributed shared
+// memory, and the scatter of a pass writes straight into the other blocks'
+// buffers; cluster barriers separate the steps, no global memory in between.
+// 20,482 primitives: 38 us, and the whole build 122 -> 90 us (65 with k_top_small).
+// Whole build by the launches / by this, with k_top_small on both: 49,153
+// primitives 123 us / 49,152 101 us; it still lost above (65,536: 126 / 144,
+// before k_top_small), hence the line.
+constexpr int kFrontBlocks = 8, kFrontThreads = 1024, kFrontItems = 6;
+constexpr uint32_t kFrontMax = kFrontBlocks * kFrontThreads * kFrontItems;  // 16 bytes a key: 96 KB a block
+
+size_t front_smem(uint32_t n) {
+  const size_t m = (n + kFrontBlocks - 1) / kFrontBlocks;
+  return 16 * m + (kFrontThreads / 32) * kBins * 2;
+}
+
+__global__ void __cluster_dims__(kFrontBlocks, 1, 1) __launch_bounds__(kFrontThreads)
+    k_front(const RtTriangle64* __restrict__ tris, const RtSphere32* __restrict__ sph, uint32_t nt, uint32_t n,
+            uint32_t mode, uint32_t* __restrict__ codes, uint32_t* __restrict__ order, uint32_t* __restrict__ clear,
+            uint32_t clear_words) {
+  namespace cg = cooperative_groups;
+  constexpr int kWarps = kFrontThreads / 32;
+  extern __shared__ uint32_t sm[];
+  __shared__ uint32_t hist[kBins], base_of[kBins], warp_sums[kBins / 32], box[6], all_box[6];
+  __shared__ float part[6][kWarps];
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t rank = cluster.block_rank(), t = threadIdx.x, lane = t & 31u, w = t >> 5;
+  const uint32_t M = (n + kFrontBlocks - 1) / kFrontBlocks;
+  const uint32_t begin = rank * M, m = begin < n ? min(M, n - begin) : 0u;
+  uint32_t *key = sm, *idx = sm + M, *key2 = sm + 2u * M, *idx2 = sm + 3u * M;
+  uint16_t* cnt = reinterpret_cast<uint16_t*>(sm + 4u * M);  // [warp][bin]
+  for (uint32_t i = rank * kFrontThreads + t; i < clear_words; i += kFrontBlocks * kFrontThreads) clear[i] = 0u;
+  // the box of the centroids (see k_centroids)
+  const bool al16 = aligned16(tris);
+  float mn[3] = {1000000000.0f, 1000000000.0f, 1000000000.0f};
+  float mx[3] = {-1000000000.0f, -1000000000.0f, -1000000000.0f};
+  for (uint32_t i = t; i < m; i += kFrontThreads) {
+    float c[3];
+    centroid(tris, sph, nt, begin + i, al16, c);
+    for (int k = 0; k < 3; ++k) {
+      mn[k] = fminf(mn[k], c[k]);
+      mx[k] = fmaxf(mx[k], c[k]);
+    }
+  }
+  for (int k = 0; k < 3; ++k) {
+    for (int o = 16; o > 0; o >>= 1) {
+      mn[k] = fminf(mn[k], __shfl_down_sync(0xFFFFFFFFu, mn[k], o));
+      mx[k] = fmaxf(mx[k], __shfl_down_sync(0xFFFFFFFFu, mx[k], o));
+    }
+    if (lane == 0u) {
+      part[k][w] = mn[k];
+      part[3 + k][w] = mx[k];
+    }
+  }
+  __syncthreads();
+  if (t < 6u) {
+    float v = part[t][0];
+    for (int k = 1; k < kWarps; ++k) v = t < 3u ? fminf(v, part[t][k]) : fmaxf(v, part[t][k]);
+    box[t] = t < 3u ? ~f2ord(v) : f2ord(v);
+  }
+  cluster.sync();
+  if (t < 6u) {
+    uint32_t v = 0u;
+    for (int r = 0; r < kFrontBlocks; ++r) v = max(v, cluster.map_shared_rank(box, r)[t]);
+    all_box[t] = v;
+  }
+  __syncthreads();
+  padded_box(all_box, mn, mx);
+  for (uint32_t i = t; i < m; i += kFrontThreads) {
+    float c[3];
+    centroid(tris, sph, nt, begin + i, al16, c);
+    key[i] = morton(c, mn, mx, mode);
+    idx[i] = begin + i;
+  }
+  // four passes of 8 bits; a warp owns a contiguous stretch of the block's keys
+  const uint32_t items = (M + kFrontThreads - 1) / kFrontThreads, first = w * 32u * items + lane;
+  for (int pass = 0; pass < 4; ++pass) {
+    const uint32_t shift = 8u * (uint32_t)pass;
+    for (uint32_t i = t; i < kWarps * kBins / 2; i += kFrontThreads) reinterpret_cast<uint32_t*>(cnt)[i] = 0u;
+    __syncthreads();
+    uint16_t rank_of[kFrontItems];
+    uint16_t* mine = cnt + w * kBins;
+#pragma unroll
+    for (int j = 0; j < kFrontItems; ++j) {
+      if ((uint32_t)j >= items) break;
+      const uint32_t i = first + 32u * j;
+      const bool ok = i < m;
+      const uint32_t d = ok ? (key[i] >> shift) & 255u : 0u;
+      uint32_t peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const bool one = (d >> b) & 1u;
+        const uint32_t ones = __ballot_sync(0xFFFFFFFFu, one);
+        peers &= one ? ones : ~ones;
+      }
+      const uint32_t seen = mine[d];
+      rank_of[j] = (uint16_t)(seen + (uint32_t)__popc(peers & ((1u << lane) - 1u)));
+      __syncwarp();
+      if (ok && lane == (uint32_t)(__ffs(peers) - 1)) mine[d] = (uint16_t)(seen + (uint32_t)__popc(peers));
+      __syncwarp();
+    }
+    __syncthreads();
+    if (t < kBins) {
+      uint32_t run = 0u;
+      for (int k = 0; k < kWarps; ++k) {
+        const uint32_t c = cnt[k * kBins + t];
+        cnt[k * kBins + t] = (uint16_t)run;
+        run += c;
+      }
+      hist[t] = run;
+    }
+    cluster.sync();
+    uint32_t total = 0u, before = 0u, scan = 0u;
+    if (t < kBins) {
+      for (uint32_t r = 0; r < (uint32_t)kFrontBlocks; ++r) {
+        const uint32_t c = cluster.map_shared_rank(hist, r)[t];
+        total += c;
+        before += r < rank ? c : 0u;
+      }
+      scan = total;  // inclusive scan over the bins
+#pragma unroll
+      for (uint32_t off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, scan, off);
+        if (lane >= off) scan += y;
+      }
+      if (lane == 31u) warp_sums[w] = scan;
+    }
+    __syncthreads();
+    if (t < kBins) {
+      for (uint32_t k = 0; k < w; ++k) scan += warp_sums[k];
+      base_of[t] = scan - total + before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kFrontItems; ++j) {
+      if ((uint32_t)j >= items) break;
+      const uint32_t i = first + 32u * j;
+      if (i < m) {
+        const uint32_t k = key[i], d = (k >> shift) & 255u;
+        const uint32_t to = base_of[d] + mine[d] + rank_of[j], r = to / M;
+        cluster.map_shared_rank(key2, r)[to - r * M] = k;
+        cluster.map_shared_rank(idx2, r)[to - r * M] = idx[i];
+      }
+    }
+    cluster.sync();
+    uint32_t* x = key; key = key2; key2 = x;
+    x = idx; idx = idx2; idx2 = x;
+  }
+  for (uint32_t i = t; i < m; i += kFrontThreads) {
+    codes[begin + i] = key[i];
+    order[begin + i] = idx[i];
+  }
+}
+
 __device__ __forceinline__ void pad_axis(float& mn, float& mx) {
   const float delta = 0.001f, padding = delta / 2.0f;
   if (mx - mn < delta) {
@@ -567,42 +726,155 @@ __device__ __forceinline__ void read_box(const RtBVHNode40* nd, float r[6]) {
   for (int k = 0; k < 6; ++k) r[k] = __ldcg(q + k);  // from L2: another SM may have written it
 }
 
+__device__ __forceinline__ void write_inner(RtBVHNode40* out, const float box[6], uint32_t left, uint32_t right) {
+  RtBVHNode40 nd;
+  nd.minX = box[0]; nd.maxX = box[1]; nd.minY = box[2]; nd.maxY = box[3]; nd.minZ = box[4]; nd.maxZ = box[5];
+  nd.left = left;
+  nd.right = right;
+  nd.primitiveIndex = 0u;
+  nd.primitiveType = 0u;
+  *out = nd;
+}
+
+// Climbs from node [l, r], whose record is written, as far as it is the second
+// to arrive, through one global slot per split.
+__device__ void climb_global(uint32_t l, uint32_t r, uint32_t n, const uint32_t* __restrict__ codes, uint32_t* slots,
+                             RtBVHNode40* nodes) {
+  const uint32_t leaf_off = n - 1u;
+  uint32_t lc = 0u, rc = 0u;
+  float box[6];
+  for (bool written = true;; written = false) {
+    const bool root = l == 0u && r == n - 1u;
+    const bool is_left = l == 0u || (r != n - 1u && delta_next(codes, r) > delta_next(codes, l - 1u));
+    const uint32_t number = root ? 0u : (l == r ? leaf_off + l : (is_left ? r : l));
+    if (written)
+      read_box(&nodes[number], box);
+    else
+      write_inner(&nodes[number], box, lc, rc);
+    if (root) break;
+    const uint32_t s = is_left ? r : l - 1u;
+    __threadfence();
+    const uint32_t other = atomicExch(&slots[s], (is_left ? l : r) + 1u);
+    if (other == 0u) break;
+    __threadfence();
+    if (is_left) r = other - 1u;
+    else l = other - 1u;
+    lc = l == s ? leaf_off + s : s;
+    rc = s + 1u == r ? leaf_off + r : s + 1u;
+    float sib[6];
+    read_box(&nodes[is_left ? rc : lc], sib);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) box[k] = (k & 1) ? fmaxf(box[k], sib[k]) : fminf(box[k], sib[k]);
+  }
+}
+
 __global__ void __launch_bounds__(128) k_top(uint32_t n, const uint32_t* __restrict__ codes,
                                              const uint2* __restrict__ open, const uint32_t* __restrict__ num_open,
                                              uint32_t* slots, RtBVHNode40* nodes) {
-  const uint32_t leaf_off = n - 1u, count = *num_open;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    uint32_t l = open[i].x, r = open[i].y, lc = 0u, rc = 0u;
-    float box[6];
-    for (bool written = true;; written = false) {
-      const bool root = l == 0u && r == n - 1u;
-      const bool is_left = l == 0u || (r != n - 1u && delta_next(codes, r) > delta_next(codes, l - 1u));
-      const uint32_t number = root ? 0u : (l == r ? leaf_off + l : (is_left ? r : l));
-      if (written) {
-        read_box(&nodes[number], box);
-      } else {
-        RtBVHNode40 nd;
-        nd.minX = box[0]; nd.maxX = box[1]; nd.minY = box[2]; nd.maxY = box[3]; nd.minZ = box[4]; nd.maxZ = box[5];
-        nd.left = lc;
-        nd.right = rc;
-        nd.primitiveIndex = 0u;
-        nd.primitiveType = 0u;
-        nodes[number] = nd;
-      }
-      if (root) break;
-      const uint32_t s = is_left ? r : l - 1u;
-      __threadfence();
-      const uint32_t other = atomicExch(&slots[s], (is_left ? l : r) + 1u);
-      if (other == 0u) break;
-      __threadfence();
-      if (is_left) r = other - 1u;
-      else l = other - 1u;
-      lc = l == s ? leaf_off + s : s;
-      rc = s + 1u == r ? leaf_off + r : s + 1u;
-      float sib[6];
-      read_box(&nodes[is_left ? rc : lc], sib);
+  const uint32_t count = *num_open;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    climb_global(open[i].x, open[i].y, n, codes, slots, nodes);
+}
+
+// The same for a small build, in one block's shared memory: the listed nodes
+// partition the sorted order, a bitmap of their first positions ranks them, and
+// k_tree's climb runs over those ranks.  A global atomic, two fences and a
+// record read per level took 45 us at 20,482 primitives; this takes 14.  A
+// list beyond kTopItems (many blocks of equal codes) climbs through the global
+// slots.
+constexpr int kTopThreads = 1024;
+constexpr uint32_t kTopItems = 2048, kTopMax = 49152;
+constexpr size_t kTopSmem = kTopItems * (12 * 4 + 4 + 4) + 8 + (kTopItems + 4) + kTopMax / 32 * 8;
+
+__global__ void __launch_bounds__(kTopThreads) k_top_small(uint32_t n, const uint32_t* __restrict__ codes,
+                                                           const uint2* __restrict__ open,
+                                                           const uint32_t* __restrict__ num_open, uint32_t* slots,
+                                                           RtBVHNode40* nodes) {
+  extern __shared__ uint32_t sm[];
+  __shared__ uint32_t warp_sums[kTopThreads / 32];
+  float* bx = reinterpret_cast<float*>(sm);           // [6][items, then internal nodes by the rank that numbers them]
+  uint32_t* slot = sm + 12 * kTopItems;               // split after rank i: 0, or a visitor's far end + 1 (and kRight)
+  uint32_t* pos = slot + kTopItems;                   // first position of rank i; n at the end
+  uint32_t* bits = pos + kTopItems + 2;               // [kTopMax / 32]
+  uint32_t* before = bits + kTopMax / 32;             // ranks before a word of bits
+  int8_t* gap = reinterpret_cast<int8_t*>(before + kTopMax / 32);  // delta across the start of rank i; -1 at the ends
+  const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5, count = *num_open, leaf_off = n - 1u;
+  if (count > kTopItems) {
+    for (uint32_t i = t; i < count; i += kTopThreads) climb_global(open[i].x, open[i].y, n, codes, slots, nodes);
+    return;
+  }
+  const uint32_t words = (n + 31u) / 32u;
+  for (uint32_t i = t; i < words; i += kTopThreads) bits[i] = 0u;
+  for (uint32_t i = t; i < count; i += kTopThreads) slot[i] = 0u;
+  __syncthreads();
+  for (uint32_t i = t; i < count; i += kTopThreads) atomicOr(&bits[open[i].x >> 5], 1u << (open[i].x & 31u));
+  __syncthreads();
+  {  // words <= 2 * kTopThreads
+    const uint32_t i = 2u * t, c0 = i < words ? (uint32_t)__popc(bits[i]) : 0u,
+                   c1 = i + 1u < words ? (uint32_t)__popc(bits[i + 1u]) : 0u;
+    uint32_t v = c0 + c1;
 #pragma unroll
-      for (int k = 0; k < 6; ++k) box[k] = (k & 1) ? fmaxf(box[k], sib[k]) : fminf(box[k], sib[k]);
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, off);
+      if (lane >= off) v += y;
+    }
+    if (lane == 31u) warp_sums[w] = v;
+    __syncthreads();
+    uint32_t base = v - c0 - c1;
+    for (uint32_t k = 0; k < w; ++k) base += warp_sums[k];
+    if (i < words) before[i] = base;
+    if (i + 1u < words) before[i + 1u] = base + c0;
+  }
+  __syncthreads();
+  for (uint32_t i = t; i < count; i += kTopThreads) {
+    const uint32_t l = open[i].x;
+    pos[before[l >> 5] + (uint32_t)__popc(bits[l >> 5] & ((1u << (l & 31u)) - 1u))] = l;
+  }
+  if (t == 0u) pos[count] = n;
+  __syncthreads();
+  for (uint32_t i = t; i <= count; i += kTopThreads)
+    gap[i] = i > 0u && i < count ? (int8_t)delta_next(codes, pos[i] - 1u) : (int8_t)-1;
+  __syncthreads();
+  for (uint32_t i = t; i < count; i += kTopThreads) {
+    uint32_t l = i, r = i;
+    int gl = gap[i], gr = gap[i + 1u];
+    float box[6];
+    {
+      const uint32_t first = pos[i], last = pos[i + 1u] - 1u;
+      read_box(&nodes[first == last ? leaf_off + first : (gr > gl ? last : first)], box);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) bx[k * 2u * kTopItems + i] = box[k];
+    }
+    for (;;) {
+      const bool is_left = gr > gl;
+      const uint32_t s = is_left ? r : l - 1u;
+      __threadfence_block();
+      const uint32_t other = atomicExch(&slot[s], is_left ? l + 1u : (r + 1u) | kRight);
+      if (other == 0u) break;
+      __threadfence_block();
+      const uint32_t end = (other & (kRight - 1u)) - 1u;
+      uint32_t sib;
+      if (is_left) {
+        sib = end == s + 1u ? end : kTopItems + s + 1u;
+        r = end;
+        gr = gap[end + 1u];
+      } else {
+        sib = end == s ? s : kTopItems + s;
+        l = end;
+        gl = gap[end];
+      }
+      const bool root = (gl & gr) < 0, left = gr > gl;
+      const uint32_t at = root ? 0u : (left ? r : l);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const float b = bx[k * 2u * kTopItems + sib];
+        box[k] = (k & 1) ? fmaxf(box[k], b) : fminf(box[k], b);
+        bx[k * 2u * kTopItems + kTopItems + at] = box[k];
+      }
+      const uint32_t first = pos[l], cut = pos[s + 1u], last = pos[r + 1u] - 1u;
+      write_inner(&nodes[root ? 0u : (left ? last : first)], box, first == cut - 1u ? leaf_off + first : cut - 1u,
+                  cut == last ? leaf_off + last : cut);
+      if (root) break;
     }
   }
 }
@@ -647,31 +919,42 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
   uint32_t* box = reinterpret_cast<uint32_t*>(p);
   uint32_t *num_open = box + kClearWords - 1, *slots = box + kClearWords;
 
-  cudaError_t e = cudaMemsetAsync(box, 0, (kClearWords + (size_t)n) * 4, st);
-  if (e != cudaSuccess) return e;
-  // the centroids take buffers that the sort's first pass does not read
-  float *cx = reinterpret_cast<float*>(va), *cy = reinterpret_cast<float*>(kb), *cz = reinterpret_cast<float*>(vb);
   const uint32_t sms = (uint32_t)device_sm_count();
-  k_centroids<<<std::min<uint32_t>((n + kT * 4 - 1) / (kT * 4), sms * 8u), kT, 0, st>>>(tris, sph, nt, n, cx, cy, cz,
-                                                                                       box);
-  k_morton<<<tiles, kT, 0, st>>>(cx, cy, cz, n, box, mode, ka, hist, tiles, tile);
   uint32_t *kin = ka, *vin = va, *kout = kb, *vout = vb;
-  for (int pass = 0; pass < 4; ++pass) {
-    const uint32_t shift = 8u * (uint32_t)pass;
-    const uint32_t* v = pass ? vin : nullptr;
-    if (pass) k_rs_hist<<<tiles, kT, 0, st>>>(kin, n, shift, hist, tiles, tile);
-    k_rs_scan<<<kBins, kT, 0, st>>>(hist, tiles, totals);
-    if (tile == kT * kItemsSmall)
-      k_rs_scatter<kItemsSmall><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
-    else
-      k_rs_scatter<kItemsLarge><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
-    std::swap(kin, kout);
-    std::swap(vin, vout);
+  cudaError_t e;
+  if (n <= kFrontMax) {
+    const size_t smem = front_smem(n);
+    e = cudaFuncSetAttribute(k_front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)front_smem(kFrontMax));
+    if (e != cudaSuccess) return e;
+    k_front<<<kFrontBlocks, kFrontThreads, smem, st>>>(tris, sph, nt, n, mode, ka, va, num_open, n + 1u);
+  } else {
+    e = cudaMemsetAsync(box, 0, (kClearWords + (size_t)n) * 4, st);
+    if (e != cudaSuccess) return e;
+    // the centroids take buffers that the sort's first pass does not read
+    float *cx = reinterpret_cast<float*>(va), *cy = reinterpret_cast<float*>(kb), *cz = reinterpret_cast<float*>(vb);
+    k_centroids<<<std::min<uint32_t>((n + kT * 4 - 1) / (kT * 4), sms * 8u), kT, 0, st>>>(tris, sph, nt, n, cx, cy, cz,
+                                                                                         box);
+    k_morton<<<tiles, kT, 0, st>>>(cx, cy, cz, n, box, mode, ka, hist, tiles, tile);
+    for (int pass = 0; pass < 4; ++pass) {
+      const uint32_t shift = 8u * (uint32_t)pass;
+      const uint32_t* v = pass ? vin : nullptr;
+      if (pass) k_rs_hist<<<tiles, kT, 0, st>>>(kin, n, shift, hist, tiles, tile);
+      k_rs_scan<<<kBins, kT, 0, st>>>(hist, tiles, totals);
+      if (tile == kT * kItemsSmall)
+        k_rs_scatter<kItemsSmall><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
+      else
+        k_rs_scatter<kItemsLarge><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
+      std::swap(kin, kout);
+      std::swap(vin, vout);
+    }
   }
   k_tree<<<blocks, kLeaves, 0, st>>>(tris, sph, nt, n, mode, kin, vin, nodes, open, num_open);
-  if (blocks > 1)
-    k_top<<<std::min<uint32_t>(blocks, sms * 16u), 128, 0, st>>>(n, kin, open, num_open, slots,
-                                                                                         nodes);
+  if (blocks > 1 && n <= kTopMax) {
+    e = cudaFuncSetAttribute(k_top_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopSmem);
+    if (e != cudaSuccess) return e;
+    k_top_small<<<1, kTopThreads, kTopSmem, st>>>(n, kin, open, num_open, slots, nodes);
+  } else if (blocks > 1)
+    k_top<<<std::min<uint32_t>(blocks, sms * 16u), 128, 0, st>>>(n, kin, open, num_open, slots, nodes);
   return cudaGetLastError();
 }
 

@@ -103,3 +103,20 @@ def test_device_build_tree_blocks(rt, cuda, n, shape):
     out = cuda.zeros((2 * n - 1) * 40 + 4, dtype=cuda.uint8, device="cuda")
     rt.build_bvh_device(raw[4:], n, d_nodes=out[4:])
     assert np.array_equal(out[4:].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 8_191, 8_193, 49_151, 49_152, 49_153])
+def test_device_build_cluster_sizes(rt, cuda, n):
+    """Sizes at the edges of the one-cluster front (blocks without keys, the last size that fits) in both modes,
+    with equal codes and with spheres among the primitives."""
+    t = rt.gen_soup(12, 0, n, 1.0, 0.01)
+    for mode in (0, 1):
+        assert np.array_equal(device_build(rt, cuda, t, mode=mode).view(np.uint8),
+                              rt.build_bvh(t, bvh_mode=mode).view(np.uint8)), mode
+    few = t[np.arange(n) * 3 // n]
+    assert np.array_equal(device_build(rt, cuda, few).view(np.uint8), rt.build_bvh(few).view(np.uint8))
+    sph = np.zeros(min(n, 50), rt.SPHERE_DTYPE)
+    sph["center"][:, :3] = np.random.default_rng(12).random((len(sph), 3)).astype(np.float32)
+    sph["radius"] = np.float32(0.02)
+    part = t[: n - len(sph)]
+    assert np.array_equal(device_build(rt, cuda, part, sph).view(np.uint8), rt.build_bvh(part, sph).view(np.uint8))
