@@ -417,6 +417,7 @@ struct WaveBufs {
 __global__ void k_wave_seed(Cam cam, uint32_t random_state, float4* __restrict__ accum, uint32_t Wd, uint32_t pix0,
                             uint32_t npix, uint32_t ns, uint32_t per_path, uint32_t* __restrict__ rng0,
                             float4* __restrict__ rays) {
+  grid_wait();
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < npix; q += gridDim.x * blockDim.x) {
     const uint32_t pix = pix0 + q;
     const uint32_t x = pix % Wd, y = pix / Wd;
@@ -468,6 +469,7 @@ __global__ void __launch_bounds__(kShadeThreads, kShadeBlocks) k_wave_shade(Devi
                              const uint2* __restrict__ hits, float4* __restrict__ next_rays,
                              uint32_t* __restrict__ next_list, uint32_t* __restrict__ cnt,
                              uint32_t* __restrict__ status_word, unsigned long long* __restrict__ stats) {
+  grid_wait();
   const uint32_t n = level == 0 ? n0 : *reinterpret_cast<volatile uint32_t*>(cnt + 4u * level + 2u);
   if (STATS && level == 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stats[0], (unsigned long long)(per_path ? n0 : npix));
   if (STATS && level > 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stats[0], (unsigned long long)n);
@@ -528,6 +530,7 @@ __global__ void __launch_bounds__(kShadeThreads, kShadeBlocks) k_wave_shade(Devi
 
 __global__ void k_wave_accum(float4* __restrict__ accum, uint32_t pix0, uint32_t npix, uint32_t ns,
                              const float4* __restrict__ color_of) {
+  grid_wait();
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < npix; q += gridDim.x * blockDim.x) {
     float4 px = accum[pix0 + q];
 #pragma unroll 8  // a 128-byte line of a thread's samples at once (41 -> 32 us)
@@ -632,7 +635,9 @@ cudaError_t launch_render_wave(const DeviceScene& S, const Cam& cam, uint32_t de
         const uint32_t np = q * ns;
         if ((e2 = cudaMemsetAsync(B.cnt, 0, 16 * ((size_t)depth + 1), cs)) != cudaSuccess) return e2;
         const uint32_t gb = std::min<uint32_t>(sms * 8, (q + 255) / 256);
-        k_wave_seed<<<gb, 256, 0, cs>>>(cam, rs, accum, Wd, pix0, q, ns, per_path, B.rng0, B.rays[0]);
+        if ((e2 = launch_dependent(k_wave_seed, gb, 256, cs, cam, rs, accum, Wd, pix0, q, ns, per_path, B.rng0,
+                                   B.rays[0])) != cudaSuccess)
+          return e2;
         for (uint32_t l = 0; l < depth; ++l) {
           const float4* r = B.rays[l & 1u];
           if ((e2 = launch_trace_raw(S, r, l == 0 ? (per_path ? np : q) : 0xFFFFFFFFu, B.hits, B.cnt + 4u * l,
@@ -640,13 +645,13 @@ cudaError_t launch_render_wave(const DeviceScene& S, const Cam& cam, uint32_t de
             return e2;
           uint32_t gs = sms * kShadeBlocks;
           if (l == 0) gs = std::min<uint32_t>(gs, (np + kShadeThreads - 1) / kShadeThreads);
-          k_wave_shade<STATS><<<gs, kShadeThreads, 0, cs>>>(S, l, depth, np, q, ns, per_path, mode, bg[0], bg[1],
-                                                            bg[2], B.color, B.gatt, B.rng0, r, B.list[l & 1u], B.hits,
-                                                            B.rays[(l + 1u) & 1u], B.list[(l + 1u) & 1u], B.cnt,
-                                                            counter + 1, stats);
+          if ((e2 = launch_dependent(k_wave_shade<STATS>, gs, kShadeThreads, cs, S, l, depth, np, q, ns, per_path, mode,
+                                     bg[0], bg[1], bg[2], B.color, B.gatt, B.rng0, r, B.list[l & 1u], B.hits,
+                                     B.rays[(l + 1u) & 1u], B.list[(l + 1u) & 1u], B.cnt, counter + 1, stats)) !=
+              cudaSuccess)
+            return e2;
         }
-        k_wave_accum<<<gb, 256, 0, cs>>>(accum, pix0, q, ns, B.color);
-        if ((e2 = cudaGetLastError()) != cudaSuccess) return e2;
+        if ((e2 = launch_dependent(k_wave_accum, gb, 256, cs, accum, pix0, q, ns, B.color)) != cudaSuccess) return e2;
       }
     }
     return cudaSuccess;
@@ -663,12 +668,14 @@ cudaError_t launch_render_wave(const DeviceScene& S, const Cam& cam, uint32_t de
 }
 
 __global__ void k_clear(float4* accum, uint32_t total) {
+  grid_wait();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
     accum[i] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
 }
 
 // SingleTriangleFullScreen.frag:13-18
 __global__ void k_resolve(const float4* accum, uint32_t total, float inv_spp_den, float4* out) {
+  grid_wait();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const float4 a = accum[i];
     float4 r;
@@ -795,8 +802,8 @@ cudaError_t launch_accum_clear(float* accum, uint32_t w, uint32_t h, void* strea
   uint32_t blocks = (total + 255u) / 256u;
   if (blocks > 4096u) blocks = 4096u;
   if (blocks == 0) return cudaSuccess;
-  k_clear<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<float4*>(accum), total);
-  return cudaGetLastError();
+  return launch_dependent(k_clear, blocks, 256, reinterpret_cast<cudaStream_t>(stream),
+                          reinterpret_cast<float4*>(accum), total);
 }
 
 cudaError_t launch_resolve(const float* accum, uint32_t w, uint32_t h, uint32_t spp, float* out, void* stream) {
@@ -804,9 +811,8 @@ cudaError_t launch_resolve(const float* accum, uint32_t w, uint32_t h, uint32_t 
   uint32_t blocks = (total + 255u) / 256u;
   if (blocks > 4096u) blocks = 4096u;
   if (blocks == 0) return cudaSuccess;
-  k_resolve<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<const float4*>(accum), total,
-                                                                        (float)spp, reinterpret_cast<float4*>(out));
-  return cudaGetLastError();
+  return launch_dependent(k_resolve, blocks, 256, reinterpret_cast<cudaStream_t>(stream),
+                          reinterpret_cast<const float4*>(accum), total, (float)spp, reinterpret_cast<float4*>(out));
 }
 
 }  // namespace rtgb

@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   }
   dev::Trav s;
   const uint32_t lane = threadIdx.x & 31u;
+  if constexpr (RAW) grid_wait();
   if (RAW && n == 0xFFFFFFFFu) n = *reinterpret_cast<volatile uint32_t*>(counter + 2);
   uint32_t ray = 0xFFFFFFFFu;
   unsigned long long vis = 0, tests = 0;
@@ -530,8 +531,8 @@ cudaError_t launch_trace_raw(const DeviceScene& S, const float4* rays, uint32_t 
   // The path tracer's bounce rays are short: refilling at 8 idle lanes beats
   // 4 there (config 2: 3.49 against 3.53 ms per frame).
   static const int refill = env_int("RT_TRACE_RAW_REFILL", 8);
-  kern<<<(uint32_t)blocks, T, 0, st>>>(S, rays, n, hits, counter, refill, stats, nullptr, spread_warps());
-  return cudaGetLastError();
+  return launch_dependent(kern, (uint32_t)blocks, T, st, S, rays, n, hits, counter, refill, stats, nullptr,
+                          spread_warps());
 }
 
 // ---- allocation-free ray queries (rt_trace_noalloc) ----

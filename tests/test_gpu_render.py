@@ -405,3 +405,33 @@ def test_deep_paths_wavefront_and_step_kernel(rt, cuda, depth):
         b = gpu_render(rt, cuda, s4, ubo, 48, 27, 2, **kw)
     assert np.array_equal(a, b)
     assert a[0::4].max() > 0.1
+
+
+@pytest.mark.parametrize("size", [(61, 37, 2), (640, 360, 3)], ids=["one_stream", "two_streams"])
+def test_frame_in_a_captured_graph(rt, cuda, size):
+    """Clear, render and resolve captured into a graph once and replayed: the frame is that of direct calls,
+    replay after replay."""
+    w, h, spp = size
+    tris, mats = lit_scene(rt)
+    ubo = rt.make_ubo((0.0, 0.5, 4.0), (0.0, 0.0, 0.0), fov=60.0, depth=5, random_state=77)
+    acc, img = (cuda.empty(w * h * 4, dtype=cuda.float32, device="cuda") for _ in range(2))
+    with rt.Scene(tris, materials=mats) as sc:
+        def frame():
+            rt.accum_clear(acc, w, h)
+            sc.render(ubo, acc, w, h, spp)
+            rt.resolve(acc, w, h, spp, img)
+
+        side = cuda.cuda.Stream()
+        with cuda.cuda.stream(side):
+            frame()  # creates the stream's workspace
+            side.synchronize()
+            want = acc.clone(), img.clone()
+            g = cuda.cuda.CUDAGraph()
+            with cuda.cuda.graph(g, stream=side):
+                frame()
+            for _ in range(3):
+                acc.fill_(-1.0)
+                img.fill_(-1.0)
+                g.replay()
+                side.synchronize()
+                assert cuda.equal(acc, want[0]) and cuda.equal(img, want[1])
