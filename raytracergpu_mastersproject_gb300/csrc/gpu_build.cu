@@ -14,6 +14,8 @@
 //   k_tree           padded leaf boxes (ConstructHLBVH.comp:117-169), internal
 //                    nodes (:72-209) and box unions, the second arriving child
 //                    continuing upward (ConstructAABBsOfInternalNodes.comp:38-64)
+//   k_mid, k_last,   the same for the nodes above k_tree's blocks
+//   k_top
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -76,6 +78,7 @@ __global__ void __launch_bounds__(kT) k_centroids(const RtTriangle64* __restrict
                                                   const RtSphere32* __restrict__ sph, uint32_t nt, uint32_t n,
                                                   float* __restrict__ cx, float* __restrict__ cy,
                                                   float* __restrict__ cz, uint32_t* __restrict__ box) {
+  grid_wait();
   constexpr int kUnroll = 4;
   __shared__ float part[6][kT / 32];
   const bool al16 = aligned16(tris);
@@ -160,6 +163,7 @@ __global__ void __launch_bounds__(kT) k_morton(const float* __restrict__ cx, con
                                                const uint32_t* __restrict__ box, uint32_t mode,
                                                uint32_t* __restrict__ codes, uint32_t* __restrict__ hist,
                                                uint32_t tiles, uint32_t tile) {
+  grid_wait();
   __shared__ uint32_t h[kBins];
   h[threadIdx.x] = 0u;
   float mn[3], mx[3];
@@ -199,6 +203,7 @@ constexpr uint32_t tile_keys(uint32_t n) { return kT * (n <= kSmallSort ? kItems
 
 __global__ void __launch_bounds__(kT) k_rs_hist(const uint32_t* __restrict__ keys, uint32_t n, uint32_t shift,
                                                 uint32_t* __restrict__ hist, uint32_t tiles, uint32_t tile) {
+  grid_wait();
   __shared__ uint32_t h[kBins];
   h[threadIdx.x] = 0u;
   __syncthreads();
@@ -246,6 +251,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t x, uint32_t* warp_sums, 
 // Block b: exclusive scan of bin b's tile counts in place, its total to totals[b].
 __global__ void __launch_bounds__(kT) k_rs_scan(uint32_t* __restrict__ hist, uint32_t tiles,
                                                 uint32_t* __restrict__ totals) {
+  grid_wait();
   __shared__ uint32_t warp_sums[kT / 32];
   uint32_t* row = hist + (size_t)blockIdx.x * tiles;
   uint32_t carry = 0;
@@ -279,6 +285,7 @@ __global__ void __launch_bounds__(kT, 4) k_rs_scatter(const uint32_t* __restrict
                                                    uint32_t n, uint32_t shift, const uint32_t* __restrict__ offs,
                                                    const uint32_t* __restrict__ totals, uint32_t tiles,
                                                    uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
+  grid_wait();
   constexpr int kWarps = kT / 32, kTile = kT * ITEMS;
   __shared__ uint32_t cnt[kWarps][kBins];
   __shared__ uint32_t sk[kTile], sv[kTile];
@@ -354,12 +361,10 @@ __global__ void __launch_bounds__(kT, 4) k_rs_scatter(const uint32_t* __restrict
 // reduced and each pass's digit counts are exchanged through distributed shared
 // memory, and the scatter of a pass writes straight into the other blocks'
 // buffers; cluster barriers separate the steps, no global memory in between.
-// 20,482 primitives: 38 us, and the whole build 122 -> 90 us (65 with k_top_small).
-// Whole build by the launches / by this, with k_top_small on both: 49,153
-// primitives 123 us / 49,152 101 us; it still lost above (65,536: 126 / 144,
-// before k_top_small), hence the line.
-constexpr int kFrontBlocks = 8, kFrontThreads = 1024, kFrontItems = 6;
-constexpr uint32_t kFrontMax = kFrontBlocks * kFrontThreads * kFrontItems;  // 16 bytes a key: 96 KB a block
+// us for the whole build by the launches / by this: 16,385 primitives 54 / 16,384
+// 49, 20,482 54 / 55, 32,769 57 / 32,768 69; hence the line.
+constexpr int kFrontBlocks = 8, kFrontThreads = 1024, kFrontItems = 2;
+constexpr uint32_t kFrontMax = kFrontBlocks * kFrontThreads * kFrontItems;  // 16 bytes a key: 32 KB a block
 
 size_t front_smem(uint32_t n) {
   const size_t m = (n + kFrontBlocks - 1) / kFrontBlocks;
@@ -370,6 +375,7 @@ __global__ void __cluster_dims__(kFrontBlocks, 1, 1) __launch_bounds__(kFrontThr
     k_front(const RtTriangle64* __restrict__ tris, const RtSphere32* __restrict__ sph, uint32_t nt, uint32_t n,
             uint32_t mode, uint32_t* __restrict__ codes, uint32_t* __restrict__ order, uint32_t* __restrict__ clear,
             uint32_t clear_words) {
+  grid_wait();
   namespace cg = cooperative_groups;
   constexpr int kWarps = kFrontThreads / 32;
   extern __shared__ uint32_t sm[];
@@ -556,10 +562,9 @@ __device__ __forceinline__ int delta_next(const uint32_t* __restrict__ codes, ui
 //
 // A block of k_tree owns kLeaves consecutive leaves.  Splits inside it meet in
 // shared memory, and its records leave as whole lines.  The few nodes whose
-// parent reaches over an edge of the block (some tens) go to a list, and k_top
-// climbs from those through global slots, reading siblings' boxes from their
-// records; climbing on in k_tree itself kept whole blocks resident for one
-// thread's chain of atomics.  The two replace a leaf pass, a pass of Karras
+// parent reaches over an edge of the block go to a list, from which k_mid and
+// k_top climb on; climbing on through global slots in k_tree itself kept whole
+// blocks resident for one thread's chain of atomics.  The two replace a leaf pass, a pass of Karras
 // searches and a bottom-up pass with a global atomic and two 40-byte record
 // reads per node.  4,194,304 triangles: 666 us for those three; k_tree 311 us as
 // one climb per thread, 260 with the climb cut in two, 195 with 8-byte stores,
@@ -567,6 +572,8 @@ __device__ __forceinline__ int delta_next(const uint32_t* __restrict__ codes, ui
 // gather, and 289 MB written); k_top 65 us of serial atomics.
 constexpr int kLeaves = 512;
 constexpr int kFirstClimb = 4;
+constexpr uint32_t kGroupBlocks = 128, kGroupLeaves = kGroupBlocks * kLeaves;  // blocks that share a list
+constexpr uint32_t kGroupOpen = kGroupLeaves + kGroupBlocks;  // at most a node per leaf and one more per block
 constexpr uint32_t kRight = 0x8000u;  // shared slot: the visitor was the right child
 // Row of the boxes in shared memory: leaves, then internal nodes; five words of
 // padding keep the ten words of neighbouring records in different banks.
@@ -578,6 +585,9 @@ __global__ void __launch_bounds__(kLeaves) k_tree(const RtTriangle64* __restrict
                                                   uint32_t mode, const uint32_t* __restrict__ codes,
                                                   const uint32_t* __restrict__ order, RtBVHNode40* __restrict__ nodes,
                                                   uint2* __restrict__ open, uint32_t* __restrict__ num_open) {
+  grid_wait();
+  open += (size_t)(blockIdx.x / kGroupBlocks) * kGroupOpen;  // the list of the block's group
+  num_open += blockIdx.x / kGroupBlocks;
   // positions are relative to the block's first leaf
   __shared__ float bx[6][kBoxRow];
   __shared__ uint32_t link[kLeaves];   // internal node: its split | kLeafLeft | kLeafRight | kLinked (0: not here)
@@ -705,7 +715,7 @@ __global__ void __launch_bounds__(kLeaves) k_tree(const RtTriangle64* __restrict
       put(out_inner + 2u * j, x, y);
     }
   }
-  // The nodes k_top climbs on from: those at the edges and the visitors that
+  // The nodes k_mid climbs on from: those at the edges and the visitors that
   // met nobody in their shared slot.
   const uint32_t tag = slot[t];
   uint32_t mine = 0u;
@@ -770,48 +780,140 @@ __device__ void climb_global(uint32_t l, uint32_t r, uint32_t n, const uint32_t*
   }
 }
 
-__global__ void __launch_bounds__(128) k_top(uint32_t n, const uint32_t* __restrict__ codes,
-                                             const uint2* __restrict__ open, const uint32_t* __restrict__ num_open,
-                                             uint32_t* slots, RtBVHNode40* nodes) {
-  const uint32_t count = *num_open;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-    climb_global(open[i].x, open[i].y, n, codes, slots, nodes);
+// One block per group of kGroupBlocks blocks of k_tree: the listed nodes
+// partition the group's positions (about nine per block of k_tree), a bitmap of
+// their first positions ranks them, and k_tree's climb runs over those ranks in
+// shared memory.  What reaches over the group's edges goes to the next list, for
+// k_last.  A group with more than kMidItems nodes (long runs of equal codes) is
+// left to k_top as it is, or, alone, climbs through the global slots here.
+// k_top alone takes a global atomic, two fences and a record read per level: 45
+// us for the top of the tree of 20,482 primitives, 14 with k_mid.
+constexpr int kMidThreads = 1024;
+constexpr uint32_t kMidItems = 1792, kMidWords = kGroupLeaves / 32;
+static_assert(kMidWords <= 2 * kMidThreads, "two words of the bitmap per thread");
+constexpr size_t kMidSmem = kMidItems * (12 * 4 + 4 + 4) + 8 + (kMidItems + 4) + kMidWords * 8;
+constexpr uint32_t kMidOpen = kMidItems + 2;  // nodes that a group leaves at most
+constexpr uint32_t kLongLists = 0x80000000u;  // in the count of those nodes: some group's list was too long
+
+// The block's shared memory in k_mid and k_last.
+struct MidShared {
+  float* bx;       // [6][nodes by rank, then internal nodes by the rank that numbers them]
+  uint32_t* slot;  // split after rank i: 0, or a visitor's far end + 1 (and kRight)
+  uint32_t* pos;   // first position of rank i; the end after the last
+  uint32_t* bits;
+  uint32_t* before;  // ranks before a word of bits
+  int8_t* gap;       // delta across the start of rank i
+};
+__device__ __forceinline__ MidShared mid_shared(uint32_t* sm) {
+  MidShared m;
+  m.bx = reinterpret_cast<float*>(sm);
+  m.slot = sm + 12 * kMidItems;
+  m.pos = m.slot + kMidItems;
+  m.bits = m.pos + kMidItems + 2;
+  m.before = m.bits + kMidWords;
+  m.gap = reinterpret_cast<int8_t*>(m.before + kMidWords);
+  return m;
 }
 
-// The same for a small build, in one block's shared memory: the listed nodes
-// partition the sorted order, a bitmap of their first positions ranks them, and
-// k_tree's climb runs over those ranks.  A global atomic, two fences and a
-// record read per level took 45 us at 20,482 primitives; this takes 14.  A
-// list beyond kTopItems (many blocks of equal codes) climbs through the global
-// slots.
-constexpr int kTopThreads = 1024;
-constexpr uint32_t kTopItems = 2048, kTopMax = 49152;
-constexpr size_t kTopSmem = kTopItems * (12 * 4 + 4 + 4) + 8 + (kTopItems + 4) + kTopMax / 32 * 8;
+// k_tree's climb over the ranks 0..count-1 (pos is set, slot is zero); nodes
+// whose sibling lies outside go to `next`.
+__device__ void climb_ranked(const MidShared& m, uint32_t count, uint32_t n, const uint32_t* __restrict__ codes,
+                             RtBVHNode40* nodes, uint2* __restrict__ next, uint32_t* __restrict__ num_next) {
+  float* bx = m.bx;
+  uint32_t *slot = m.slot, *pos = m.pos;
+  int8_t* gap = m.gap;
+  const uint32_t t = threadIdx.x, leaf_off = n - 1u;
+  for (uint32_t i = t; i <= count; i += kMidThreads)
+    gap[i] = pos[i] > 0u && pos[i] < n ? (int8_t)delta_next(codes, pos[i] - 1u) : (int8_t)-1;
+  __syncthreads();
+  for (uint32_t i = t; i < count; i += kMidThreads) {
+    uint32_t l = i, r = i;
+    int gl = gap[i], gr = gap[i + 1u];
+    float box[6];
+    {
+      const uint32_t first = pos[i], last = pos[i + 1u] - 1u;
+      read_box(&nodes[first == last ? leaf_off + first : (gr > gl ? last : first)], box);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) bx[k * 2u * kMidItems + i] = box[k];
+    }
+    for (;;) {
+      const bool is_left = gr > gl;
+      const uint32_t s = is_left ? r : l - 1u;
+      if (is_left ? r == count - 1u : l == 0u) {  // the sibling is in another group
+        next[atomicAdd(num_next, 1u) & ~kLongLists] = make_uint2(pos[l], pos[r + 1u] - 1u);
+        break;
+      }
+      __threadfence_block();
+      const uint32_t other = atomicExch(&slot[s], is_left ? l + 1u : (r + 1u) | kRight);
+      if (other == 0u) break;
+      __threadfence_block();
+      slot[s] = 0u;
+      const uint32_t far = (other & (kRight - 1u)) - 1u;
+      uint32_t sib;
+      if (is_left) {
+        sib = far == s + 1u ? far : kMidItems + s + 1u;
+        r = far;
+        gr = gap[far + 1u];
+      } else {
+        sib = far == s ? s : kMidItems + s;
+        l = far;
+        gl = gap[far];
+      }
+      const bool root = (gl & gr) < 0, left = gr > gl;
+      const uint32_t at = root ? 0u : (left ? r : l);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const float b = bx[k * 2u * kMidItems + sib];
+        box[k] = (k & 1) ? fmaxf(box[k], b) : fminf(box[k], b);
+        bx[k * 2u * kMidItems + kMidItems + at] = box[k];
+      }
+      const uint32_t first = pos[l], cut = pos[s + 1u], last = pos[r + 1u] - 1u;
+      write_inner(&nodes[root ? 0u : (left ? last : first)], box, first == cut - 1u ? leaf_off + first : cut - 1u,
+                  cut == last ? leaf_off + last : cut);
+      if (root) break;
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = t; i < count; i += kMidThreads) {  // visitors that met nobody
+    const uint32_t tag = slot[i];
+    if (tag == 0u) continue;
+    const uint32_t far = (tag & (kRight - 1u)) - 1u;
+    const uint32_t l = (tag & kRight) ? i + 1u : far, r = (tag & kRight) ? far : i;
+    next[atomicAdd(num_next, 1u) & ~kLongLists] = make_uint2(pos[l], pos[r + 1u] - 1u);
+  }
+}
 
-__global__ void __launch_bounds__(kTopThreads) k_top_small(uint32_t n, const uint32_t* __restrict__ codes,
-                                                           const uint2* __restrict__ open,
-                                                           const uint32_t* __restrict__ num_open, uint32_t* slots,
-                                                           RtBVHNode40* nodes) {
+__global__ void __launch_bounds__(kMidThreads) k_mid(uint32_t n, const uint32_t* __restrict__ codes,
+                                                     const uint2* __restrict__ open,
+                                                     const uint32_t* __restrict__ num_open, uint32_t* slots,
+                                                     RtBVHNode40* nodes, uint2* __restrict__ next,
+                                                     uint32_t* __restrict__ num_next) {
+  grid_wait();
   extern __shared__ uint32_t sm[];
-  __shared__ uint32_t warp_sums[kTopThreads / 32];
-  float* bx = reinterpret_cast<float*>(sm);           // [6][items, then internal nodes by the rank that numbers them]
-  uint32_t* slot = sm + 12 * kTopItems;               // split after rank i: 0, or a visitor's far end + 1 (and kRight)
-  uint32_t* pos = slot + kTopItems;                   // first position of rank i; n at the end
-  uint32_t* bits = pos + kTopItems + 2;               // [kTopMax / 32]
-  uint32_t* before = bits + kTopMax / 32;             // ranks before a word of bits
-  int8_t* gap = reinterpret_cast<int8_t*>(before + kTopMax / 32);  // delta across the start of rank i; -1 at the ends
-  const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5, count = *num_open, leaf_off = n - 1u;
-  if (count > kTopItems) {
-    for (uint32_t i = t; i < count; i += kTopThreads) climb_global(open[i].x, open[i].y, n, codes, slots, nodes);
+  __shared__ uint32_t warp_sums[kMidThreads / 32];
+  const MidShared m = mid_shared(sm);
+  uint32_t *slot = m.slot, *pos = m.pos, *bits = m.bits, *before = m.before;
+  const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
+  const uint32_t base = blockIdx.x * kGroupLeaves, end = min(n, base + kGroupLeaves);
+  const uint32_t count = num_open[blockIdx.x];
+  open += (size_t)blockIdx.x * kGroupOpen;
+  if (count > kMidItems) {
+    if (gridDim.x == 1u)
+      for (uint32_t i = t; i < count; i += kMidThreads) climb_global(open[i].x, open[i].y, n, codes, slots, nodes);
+    else if (t == 0u)
+      atomicOr(num_next, kLongLists);
     return;
   }
-  const uint32_t words = (n + 31u) / 32u;
-  for (uint32_t i = t; i < words; i += kTopThreads) bits[i] = 0u;
-  for (uint32_t i = t; i < count; i += kTopThreads) slot[i] = 0u;
+  const uint32_t words = (end - base + 31u) / 32u;
+  for (uint32_t i = t; i < words; i += kMidThreads) bits[i] = 0u;
+  for (uint32_t i = t; i < count; i += kMidThreads) slot[i] = 0u;
   __syncthreads();
-  for (uint32_t i = t; i < count; i += kTopThreads) atomicOr(&bits[open[i].x >> 5], 1u << (open[i].x & 31u));
+  for (uint32_t i = t; i < count; i += kMidThreads) {
+    const uint32_t l = open[i].x - base;
+    atomicOr(&bits[l >> 5], 1u << (l & 31u));
+  }
   __syncthreads();
-  {  // words <= 2 * kTopThreads
+  {
     const uint32_t i = 2u * t, c0 = i < words ? (uint32_t)__popc(bits[i]) : 0u,
                    c1 = i + 1u < words ? (uint32_t)__popc(bits[i + 1u]) : 0u;
     uint32_t v = c0 + c1;
@@ -822,75 +924,88 @@ __global__ void __launch_bounds__(kTopThreads) k_top_small(uint32_t n, const uin
     }
     if (lane == 31u) warp_sums[w] = v;
     __syncthreads();
-    uint32_t base = v - c0 - c1;
-    for (uint32_t k = 0; k < w; ++k) base += warp_sums[k];
-    if (i < words) before[i] = base;
-    if (i + 1u < words) before[i + 1u] = base + c0;
+    uint32_t b = v - c0 - c1;
+    for (uint32_t k = 0; k < w; ++k) b += warp_sums[k];
+    if (i < words) before[i] = b;
+    if (i + 1u < words) before[i + 1u] = b + c0;
   }
   __syncthreads();
-  for (uint32_t i = t; i < count; i += kTopThreads) {
-    const uint32_t l = open[i].x;
-    pos[before[l >> 5] + (uint32_t)__popc(bits[l >> 5] & ((1u << (l & 31u)) - 1u))] = l;
+  for (uint32_t i = t; i < count; i += kMidThreads) {
+    const uint32_t l = open[i].x - base;
+    pos[before[l >> 5] + (uint32_t)__popc(bits[l >> 5] & ((1u << (l & 31u)) - 1u))] = base + l;
   }
-  if (t == 0u) pos[count] = n;
+  if (t == 0u) pos[count] = end;
   __syncthreads();
-  for (uint32_t i = t; i <= count; i += kTopThreads)
-    gap[i] = i > 0u && i < count ? (int8_t)delta_next(codes, pos[i] - 1u) : (int8_t)-1;
-  __syncthreads();
-  for (uint32_t i = t; i < count; i += kTopThreads) {
-    uint32_t l = i, r = i;
-    int gl = gap[i], gr = gap[i + 1u];
-    float box[6];
-    {
-      const uint32_t first = pos[i], last = pos[i + 1u] - 1u;
-      read_box(&nodes[first == last ? leaf_off + first : (gr > gl ? last : first)], box);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) bx[k * 2u * kTopItems + i] = box[k];
-    }
-    for (;;) {
-      const bool is_left = gr > gl;
-      const uint32_t s = is_left ? r : l - 1u;
-      __threadfence_block();
-      const uint32_t other = atomicExch(&slot[s], is_left ? l + 1u : (r + 1u) | kRight);
-      if (other == 0u) break;
-      __threadfence_block();
-      const uint32_t end = (other & (kRight - 1u)) - 1u;
-      uint32_t sib;
-      if (is_left) {
-        sib = end == s + 1u ? end : kTopItems + s + 1u;
-        r = end;
-        gr = gap[end + 1u];
-      } else {
-        sib = end == s ? s : kTopItems + s;
-        l = end;
-        gl = gap[end];
-      }
-      const bool root = (gl & gr) < 0, left = gr > gl;
-      const uint32_t at = root ? 0u : (left ? r : l);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const float b = bx[k * 2u * kTopItems + sib];
-        box[k] = (k & 1) ? fmaxf(box[k], b) : fminf(box[k], b);
-        bx[k * 2u * kTopItems + kTopItems + at] = box[k];
-      }
-      const uint32_t first = pos[l], cut = pos[s + 1u], last = pos[r + 1u] - 1u;
-      write_inner(&nodes[root ? 0u : (left ? last : first)], box, first == cut - 1u ? leaf_off + first : cut - 1u,
-                  cut == last ? leaf_off + last : cut);
-      if (root) break;
-    }
-  }
+  climb_ranked(m, count, n, codes, nodes, next, num_next);
 }
+
+// The top of a tree of several groups: the nodes that k_mid's groups left, about
+// ten each, ranked by counting, in one block.  Leaves the work to k_top when they
+// are too many or some group's list was too long.
+__device__ __forceinline__ bool fits_last(uint32_t num_next) { return num_next <= kMidItems; }
+
+__global__ void __launch_bounds__(kMidThreads) k_last(uint32_t n, const uint32_t* __restrict__ codes,
+                                                      uint2* __restrict__ next, uint32_t* __restrict__ num_next,
+                                                      RtBVHNode40* nodes) {
+  grid_wait();
+  extern __shared__ uint32_t sm[];
+  const MidShared m = mid_shared(sm);
+  const uint32_t t = threadIdx.x, count = *num_next;
+  if (!fits_last(count)) return;
+  uint32_t* first = m.slot;  // unranked, until the ranks are known
+  for (uint32_t i = t; i < count; i += kMidThreads) first[i] = next[i].x;
+  __syncthreads();
+  for (uint32_t i = t; i < count; i += kMidThreads) {
+    const uint32_t l = first[i];
+    uint32_t rank = 0u;
+    for (uint32_t j = 0; j < count; ++j) rank += first[j] < l ? 1u : 0u;
+    m.pos[rank] = l;
+  }
+  if (t == 0u) m.pos[count] = n;
+  __syncthreads();
+  for (uint32_t i = t; i < count; i += kMidThreads) m.slot[i] = 0u;
+  __syncthreads();
+  climb_ranked(m, count, n, codes, nodes, next, num_next);
+}
+
+// One global slot per split: all of k_tree's lists (`all`), or what k_last left.
+// blockIdx.y: the group.
+__global__ void __launch_bounds__(128) k_top(uint32_t n, const uint32_t* __restrict__ codes,
+                                             const uint2* __restrict__ open, const uint32_t* __restrict__ num_open,
+                                             const uint2* __restrict__ next, const uint32_t* __restrict__ num_next,
+                                             bool all, uint32_t* slots, RtBVHNode40* nodes) {
+  grid_wait();
+  if (!all && fits_last(*num_next)) return;
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  if (!all && blockIdx.y == 0u) {
+    const uint32_t count = *num_next & ~kLongLists;
+    for (uint32_t i = t; i < count; i += step) climb_global(next[i].x, next[i].y, n, codes, slots, nodes);
+  }
+  const uint32_t c = num_open[blockIdx.y];
+  if (!all && c <= kMidItems) return;
+  open += (size_t)blockIdx.y * kGroupOpen;
+  for (uint32_t i = t; i < c; i += step) climb_global(open[i].x, open[i].y, n, codes, slots, nodes);
+}
+
+// Groups up to which k_mid and k_last finish the tree.  us for the whole build
+// with them / with k_top over all lists: 262,144 primitives (4 groups) 91 / 102,
+// 1,000,000 (16) 176 / 189, 2,000,000 (31) 275 / 289, 3,000,000 (46) 376 / 384,
+// 4,194,304 (64) 501 / 489.
+constexpr uint32_t kLastGroups = 48;
 
 }  // namespace
 
 // Cleared at the start: the centroid box (six words, two unused), the count of
-// k_tree's list, then a slot per split.
+// k_mid's list, those of k_tree's lists, then a slot per split.
 constexpr size_t kClearWords = 9;
+
+constexpr uint32_t tree_groups(uint32_t n) { return (n + kGroupLeaves - 1) / kGroupLeaves; }
 
 size_t device_build_scratch_bytes(uint32_t n) {
   const uint32_t tiles = (n + tile_keys(n) - 1) / tile_keys(n);
-  const uint32_t blocks = (n + kLeaves - 1) / kLeaves;
-  return 16 + kBins * 4 + (size_t)n * 4 * 4 + (size_t)blocks * 8 + (size_t)kBins * tiles * 4 + kClearWords * 4 + (size_t)n * 4;
+  const size_t blocks = (n + kLeaves - 1) / kLeaves, groups = tree_groups(n);
+  return 24 + kBins * 4 + (size_t)n * 4 * 4 + blocks * 8 + groups * kMidOpen * 8 + (size_t)kBins * tiles * 4 +
+         (kClearWords + groups + (size_t)n) * 4;
 }
 
 // nodes: 2n-1 records; scratch: device_build_scratch_bytes(n).
@@ -913,13 +1028,16 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
   p += (size_t)n * 4;
   uint32_t* vb = reinterpret_cast<uint32_t*>(p);
   p += (size_t)n * 4;
-  const uint32_t blocks = (n + kLeaves - 1) / kLeaves;
+  const uint32_t blocks = (n + kLeaves - 1) / kLeaves, groups = tree_groups(n);
   p += (size_t)blocks * 8;
+  uint2* next = reinterpret_cast<uint2*>((reinterpret_cast<uintptr_t>(p) + 7) & ~(uintptr_t)7);
+  p = reinterpret_cast<char*>(next + (size_t)groups * kMidOpen);
   const uint32_t tile = tile_keys(n), tiles = (n + tile - 1) / tile;
   uint32_t* hist = reinterpret_cast<uint32_t*>(p);
   p += (size_t)kBins * tiles * 4;
   uint32_t* box = reinterpret_cast<uint32_t*>(p);
-  uint32_t *num_open = box + kClearWords - 1, *slots = box + kClearWords;
+  uint32_t *num_next = box + kClearWords - 1, *num_open = num_next + 1, *slots = num_open + groups;
+  const uint32_t cleared = 1u + groups + n;  // from num_next on
 
   const uint32_t sms = (uint32_t)device_sm_count();
   uint32_t *kin = ka, *vin = va, *kout = kb, *vout = vb;
@@ -928,36 +1046,45 @@ cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtS
     const size_t smem = front_smem(n);
     e = cudaFuncSetAttribute(k_front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)front_smem(kFrontMax));
     if (e != cudaSuccess) return e;
-    k_front<<<kFrontBlocks, kFrontThreads, smem, st>>>(tris, sph, nt, n, mode, ka, va, num_open, n + 1u);
+    e = launch_dependent(k_front, kFrontBlocks, kFrontThreads, smem, st, tris, sph, nt, n, mode, ka, va, num_next, cleared);
+    if (e != cudaSuccess) return e;
   } else {
-    e = cudaMemsetAsync(box, 0, (kClearWords + (size_t)n) * 4, st);
+    e = cudaMemsetAsync(box, 0, (kClearWords - 1 + (size_t)cleared) * 4, st);
     if (e != cudaSuccess) return e;
     // the centroids take buffers that the sort's first pass does not read
     float *cx = reinterpret_cast<float*>(va), *cy = reinterpret_cast<float*>(kb), *cz = reinterpret_cast<float*>(vb);
-    k_centroids<<<std::min<uint32_t>((n + kT * 4 - 1) / (kT * 4), sms * 8u), kT, 0, st>>>(tris, sph, nt, n, cx, cy, cz,
-                                                                                         box);
-    k_morton<<<tiles, kT, 0, st>>>(cx, cy, cz, n, box, mode, ka, hist, tiles, tile);
-    for (int pass = 0; pass < 4; ++pass) {
+    e = launch_dependent(k_centroids, std::min<uint32_t>((n + kT * 4 - 1) / (kT * 4), sms * 8u), kT, 0, st, tris, sph, nt,
+                         n, cx, cy, cz, box);
+    if (e == cudaSuccess)
+      e = launch_dependent(k_morton, tiles, kT, 0, st, cx, cy, cz, n, box, mode, ka, hist, tiles, tile);
+    for (int pass = 0; pass < 4 && e == cudaSuccess; ++pass) {
       const uint32_t shift = 8u * (uint32_t)pass;
       const uint32_t* v = pass ? vin : nullptr;
-      if (pass) k_rs_hist<<<tiles, kT, 0, st>>>(kin, n, shift, hist, tiles, tile);
-      k_rs_scan<<<kBins, kT, 0, st>>>(hist, tiles, totals);
-      if (tile == kT * kItemsSmall)
-        k_rs_scatter<kItemsSmall><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
-      else
-        k_rs_scatter<kItemsLarge><<<tiles, kT, 0, st>>>(kin, v, n, shift, hist, totals, tiles, kout, vout);
+      if (pass) e = launch_dependent(k_rs_hist, tiles, kT, 0, st, kin, n, shift, hist, tiles, tile);
+      if (e == cudaSuccess) e = launch_dependent(k_rs_scan, kBins, kT, 0, st, hist, tiles, totals);
+      if (e == cudaSuccess)
+        e = launch_dependent(tile == kT * kItemsSmall ? k_rs_scatter<kItemsSmall> : k_rs_scatter<kItemsLarge>, tiles, kT,
+                             0, st, kin, v, n, shift, hist, totals, tiles, kout, vout);
       std::swap(kin, kout);
       std::swap(vin, vout);
     }
-  }
-  k_tree<<<blocks, kLeaves, 0, st>>>(tris, sph, nt, n, mode, kin, vin, nodes, open, num_open);
-  if (blocks > 1 && n <= kTopMax) {
-    e = cudaFuncSetAttribute(k_top_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopSmem);
     if (e != cudaSuccess) return e;
-    k_top_small<<<1, kTopThreads, kTopSmem, st>>>(n, kin, open, num_open, slots, nodes);
-  } else if (blocks > 1)
-    k_top<<<std::min<uint32_t>(blocks, sms * 16u), 128, 0, st>>>(n, kin, open, num_open, slots, nodes);
-  return cudaGetLastError();
+  }
+  e = launch_dependent(k_tree, blocks, kLeaves, 0, st, tris, sph, nt, n, mode, kin, vin, nodes, open, num_open);
+  if (e == cudaSuccess && blocks > 1 && groups <= kLastGroups) {
+    e = cudaFuncSetAttribute(k_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmem);
+    if (e == cudaSuccess)
+      e = launch_dependent(k_mid, groups, kMidThreads, kMidSmem, st, n, kin, open, num_open, slots, nodes, next,
+                           num_next);
+    if (e == cudaSuccess && groups > 1)
+      e = cudaFuncSetAttribute(k_last, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmem);
+    if (e == cudaSuccess && groups > 1)
+      e = launch_dependent(k_last, 1, kMidThreads, kMidSmem, st, n, kin, next, num_next, nodes);
+  }
+  if (e == cudaSuccess && groups > 1)
+    e = launch_dependent(k_top, dim3(16, groups), 128, 0, st, n, kin, open, num_open, next, num_next,
+                         groups > kLastGroups, slots, nodes);
+  return e;
 }
 
 }  // namespace rtgb

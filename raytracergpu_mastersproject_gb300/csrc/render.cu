@@ -635,7 +635,7 @@ cudaError_t launch_render_wave(const DeviceScene& S, const Cam& cam, uint32_t de
         const uint32_t np = q * ns;
         if ((e2 = cudaMemsetAsync(B.cnt, 0, 16 * ((size_t)depth + 1), cs)) != cudaSuccess) return e2;
         const uint32_t gb = std::min<uint32_t>(sms * 8, (q + 255) / 256);
-        if ((e2 = launch_dependent(k_wave_seed, gb, 256, cs, cam, rs, accum, Wd, pix0, q, ns, per_path, B.rng0,
+        if ((e2 = launch_dependent(k_wave_seed, gb, 256, 0, cs, cam, rs, accum, Wd, pix0, q, ns, per_path, B.rng0,
                                    B.rays[0])) != cudaSuccess)
           return e2;
         for (uint32_t l = 0; l < depth; ++l) {
@@ -645,13 +645,13 @@ cudaError_t launch_render_wave(const DeviceScene& S, const Cam& cam, uint32_t de
             return e2;
           uint32_t gs = sms * kShadeBlocks;
           if (l == 0) gs = std::min<uint32_t>(gs, (np + kShadeThreads - 1) / kShadeThreads);
-          if ((e2 = launch_dependent(k_wave_shade<STATS>, gs, kShadeThreads, cs, S, l, depth, np, q, ns, per_path, mode,
+          if ((e2 = launch_dependent(k_wave_shade<STATS>, gs, kShadeThreads, 0, cs, S, l, depth, np, q, ns, per_path, mode,
                                      bg[0], bg[1], bg[2], B.color, B.gatt, B.rng0, r, B.list[l & 1u], B.hits,
                                      B.rays[(l + 1u) & 1u], B.list[(l + 1u) & 1u], B.cnt, counter + 1, stats)) !=
               cudaSuccess)
             return e2;
         }
-        if ((e2 = launch_dependent(k_wave_accum, gb, 256, cs, accum, pix0, q, ns, B.color)) != cudaSuccess) return e2;
+        if ((e2 = launch_dependent(k_wave_accum, gb, 256, 0, cs, accum, pix0, q, ns, B.color)) != cudaSuccess) return e2;
       }
     }
     return cudaSuccess;
@@ -802,7 +802,7 @@ cudaError_t launch_accum_clear(float* accum, uint32_t w, uint32_t h, void* strea
   uint32_t blocks = (total + 255u) / 256u;
   if (blocks > 4096u) blocks = 4096u;
   if (blocks == 0) return cudaSuccess;
-  return launch_dependent(k_clear, blocks, 256, reinterpret_cast<cudaStream_t>(stream),
+  return launch_dependent(k_clear, blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream),
                           reinterpret_cast<float4*>(accum), total);
 }
 
@@ -811,7 +811,7 @@ cudaError_t launch_resolve(const float* accum, uint32_t w, uint32_t h, uint32_t 
   uint32_t blocks = (total + 255u) / 256u;
   if (blocks > 4096u) blocks = 4096u;
   if (blocks == 0) return cudaSuccess;
-  return launch_dependent(k_resolve, blocks, 256, reinterpret_cast<cudaStream_t>(stream),
+  return launch_dependent(k_resolve, blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream),
                           reinterpret_cast<const float4*>(accum), total, (float)spp, reinterpret_cast<float4*>(out));
 }
 

@@ -79,13 +79,15 @@ struct NvtxRange {
 // has started, griddepcontrol.launch_dependents, holds places that the other
 // stream's blocks need: 105 and 2,964 us.)
 template <class... P, class... A>
-cudaError_t launch_dependent(void (*k)(P...), uint32_t grid, uint32_t block, cudaStream_t st, A&&... args) {
+cudaError_t launch_dependent(void (*k)(P...), dim3 grid, uint32_t block, size_t smem, cudaStream_t st,
+                             A&&... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;

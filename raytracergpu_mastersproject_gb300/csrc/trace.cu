@@ -531,7 +531,7 @@ cudaError_t launch_trace_raw(const DeviceScene& S, const float4* rays, uint32_t 
   // The path tracer's bounce rays are short: refilling at 8 idle lanes beats
   // 4 there (config 2: 3.49 against 3.53 ms per frame).
   static const int refill = env_int("RT_TRACE_RAW_REFILL", 8);
-  return launch_dependent(kern, (uint32_t)blocks, T, st, S, rays, n, hits, counter, refill, stats, nullptr,
+  return launch_dependent(kern, (uint32_t)blocks, T, 0, st, S, rays, n, hits, counter, refill, stats, nullptr,
                           spread_warps());
 }
 

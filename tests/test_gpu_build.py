@@ -1,6 +1,8 @@
 """The GPU LBVH build (rt_build_bvh_device) must emit exactly the node array
 of the oracle's transcription of the six S1 passes (ModelSpaceToWorldSpace.comp
 to ConstructAABBsOfInternalNodes.comp), and of the host build."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -75,7 +77,7 @@ def test_device_build_matches_oracle(rt, orc, cuda, mode):
                           orc.build_bvh(big, mode=mode)[0].view(np.uint8))
 
 
-@pytest.mark.parametrize("n", [1024, 1025, 1_048_576, 1_048_577, 1_052_673])
+@pytest.mark.parametrize("n", [1024, 1025, 1_048_576, 1_048_577, 1_052_673, 3_145_728, 3_145_729])
 def test_device_build_sort_tiles(rt, cuda, n):
     """Sizes at the edges of the radix sort's tiles and where its tile size changes, for scattered codes and
     for a few long runs of equal ones."""
@@ -85,7 +87,7 @@ def test_device_build_sort_tiles(rt, cuda, n):
     assert np.array_equal(device_build(rt, cuda, runs).view(np.uint8), rt.build_bvh(runs).view(np.uint8))
 
 
-@pytest.mark.parametrize("n", [511, 512, 513, 1024, 1537, 40_961])
+@pytest.mark.parametrize("n", [511, 512, 513, 1024, 1537, 40_961, 65_536, 65_537, 131_073, 300_001])
 @pytest.mark.parametrize("shape", ["soup", "equal", "line"])
 def test_device_build_tree_blocks(rt, cuda, n, shape):
     """Sizes at the edges of the tree kernel's blocks: shallow trees, one code everywhere (the index decides)
@@ -105,7 +107,7 @@ def test_device_build_tree_blocks(rt, cuda, n, shape):
     assert np.array_equal(out[4:].cpu().numpy(), want)
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 8_191, 8_193, 49_151, 49_152, 49_153])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 8_191, 8_193, 16_383, 16_384, 16_385])
 def test_device_build_cluster_sizes(rt, cuda, n):
     """Sizes at the edges of the one-cluster front (blocks without keys, the last size that fits) in both modes,
     with equal codes and with spheres among the primitives."""
@@ -145,3 +147,22 @@ def test_device_build_scratch_is_given_back(rt, cuda):
     rt.release_stream()
     assert free0 - cuda.cuda.mem_get_info()[0] <= 4 << 20
     assert np.array_equal(d_n[0].cpu().numpy(), want[0])
+
+
+@pytest.mark.parametrize("part", ["all", "one_group"])
+def test_device_build_long_lists(rt, cuda, part):
+    """Codes with at most five bits set: deep one-sided subtrees everywhere, so that a group of blocks leaves more
+    nodes for the top of the tree than one block takes (1,850 of 174,438 primitives' middle group, 1,870 of
+    65,536 primitives in one group; the limit is 1,792)."""
+    codes = np.array(sorted([0] + [sum(1 << b for b in c) for k in range(1, 6)
+                                   for c in itertools.combinations(range(30), k)]), np.int64)
+    q = np.zeros((len(codes), 3))
+    for b in range(30):
+        q[:, b % 3] += ((codes >> b) & 1) * (1 << (b // 3))
+    if part == "one_group":
+        q = np.concatenate([q[:1], q[70_000:70_000 + 65_534]])
+    centre = np.concatenate([(q + 0.5) / 1024, [[1.0 - 0.4 / 1024] * 3]]).astype(np.float32)
+    t = np.zeros(len(centre), rt.TRIANGLE_DTYPE)
+    for v, d in (("v0", (-1, 0, 0)), ("v1", (0.5, 1, 0)), ("v2", (0.5, -1, 0))):
+        t[v][:, :3] = centre + np.float32(1e-5) * np.array(d, np.float32)
+    assert np.array_equal(device_build(rt, cuda, t).view(np.uint8), rt.build_bvh(t).view(np.uint8))
