@@ -687,8 +687,12 @@ rt_status rt_trace_host(rt_scene* scene, const RtRay* h_rays, uint32_t n, RtHit*
   // larger.
   //
   // Hits are staged in device memory and downloaded per chunk on a third
-  // stream; chunks start at 2 Mi rays and grow 4x, and the plan ends with a
-  // small chunk, so that the one download that overlaps nothing is short.
+  // stream; chunks start at 512 Ki rays (256 Ki below 2 Mi rays) and grow 4x,
+  // and the plan ends with a small chunk, so that the one download that overlaps
+  // nothing is short.  us per call by first chunk, 256 Ki / 512 Ki / 2 Mi: 1.2 M
+  // rays on 524,288 triangles 888 / 997 / 891, 3 M 1,769 / 1,763 / 2,044, 8 M
+  // 4,355 / 4,123 / 4,297, 16 M 8,073 / 8,217 / 8,277; on 4,194,304 triangles
+  // 3 M 2,321 / 2,241 / 2,752, 16.8 M 10,228 / 10,228 / 10,238.
   // With RT_HOST_DIRECT_HITS=1 and page-locked h_hits the kernels instead
   // write the hits there directly over the host link (scattered 8-byte
   // stores, overlapped with tracing) and chunks grow 8x; on GB300 that
@@ -697,7 +701,7 @@ rt_status rt_trace_host(rt_scene* scene, const RtRay* h_rays, uint32_t n, RtHit*
   static const uint32_t kFirstChunk = [] {
     const char* e = std::getenv("RT_HOST_FIRST_CHUNK_RAYS");
     const long v = e ? std::atol(e) : 0;
-    return v >= 4096 && v <= (1l << 30) ? (uint32_t)v : (1u << 21);
+    return v >= 4096 && v <= (1l << 30) ? (uint32_t)v : 0u;
   }();
   static const uint32_t kLastChunk = [] {
     const char* e = std::getenv("RT_HOST_LAST_CHUNK_RAYS");
@@ -724,6 +728,7 @@ rt_status rt_trace_host(rt_scene* scene, const RtRay* h_rays, uint32_t n, RtHit*
     return v >= 2 && v <= 64 ? (uint32_t)v : 0u;
   }();
   const uint32_t growth = kGrowth ? kGrowth : (direct ? 8u : 4u);
+  const uint32_t first_chunk = kFirstChunk ? kFirstChunk : (direct ? 1u << 21 : n < (1u << 21) ? 1u << 18 : 1u << 19);
   const uint32_t chunk = std::min<uint32_t>(n, direct ? (1u << 24) : (1u << 23));  // buffer capacity
   // each half's rays and hits start 256-byte aligned: straight after an odd number of 8-byte hits the second
   // half's rays would be off the 16 bytes that the kernels load them by
@@ -771,7 +776,7 @@ rt_status rt_trace_host(rt_scene* scene, const RtRay* h_rays, uint32_t n, RtHit*
   if ((e = cudaStreamWaitEvent(w->copy_in, w->ev[6], 0)) != cudaSuccess) return drain(cuda_fail(e, "wait"));
   uint32_t chunks = 0;
   auto enqueue = [&]() -> rt_status {
-    uint32_t size = std::min(chunk, kFirstChunk);
+    uint32_t size = std::min(chunk, first_chunk);
     for (uint32_t c = 0, off = 0, cnt = 0; off < n;
          ++c, off += cnt, size = (uint32_t)std::min<uint64_t>((uint64_t)growth * size, chunk)) {
       const uint32_t b = c & 1u;
