@@ -639,7 +639,7 @@ def run_ours(args):
                "block_ms_per_step": [round(b * 1e3, 3) for b in blocks],
                "timing": f"wall clock around each of 3 blocks of {k} calls after {max(3, args.warmup)} warm-up "
                          "calls; the median block",
-               "path": "rt_trace_host, pinned host buffers: rays in chunks of 2 Mi, 8 Mi, the rest but "
+               "path": "rt_trace_host, pinned host buffers: rays in chunks of 512 Ki, 2 Mi, 8 Mi, the rest but "
                        "512 Ki, and 512 Ki, each uploaded on a copy stream while the one before traces (two trace "
                        "streams); hits staged in HBM and downloaded per chunk on a third stream"}
         hits_dev = d_hits.cpu().numpy().view(rt.HIT_DTYPE)
