@@ -878,7 +878,9 @@ static rt_status render_impl(rt_scene* scene, const RtRaytraceUBO* ubo, float* d
       w->wave_bytes = need;
     }
   }
-  cudaError_t e = cudaMemsetAsync(w->counters, 0, (h_counts ? 16 : 2) * sizeof(uint32_t), st);
+  // the pixel queue of the other schedules, and the work counters
+  cudaError_t e = cudaSuccess;
+  if (h_counts || !wave_paths) e = cudaMemsetAsync(w->counters, 0, (h_counts ? 16 : 2) * sizeof(uint32_t), st);
   if (e != cudaSuccess) return cuda_fail(e, "rt_render: memset");
   unsigned long long* stats = h_counts ? reinterpret_cast<unsigned long long*>(w->counters + 8) : nullptr;
   const uint32_t mode = (o.shade_mode == RT_SHADE_EXTENDED ? kRenderExtended : 0u) |

@@ -416,8 +416,12 @@ struct WaveBufs {
 
 __global__ void k_wave_seed(Cam cam, uint32_t random_state, float4* __restrict__ accum, uint32_t Wd, uint32_t pix0,
                             uint32_t npix, uint32_t ns, uint32_t per_path, uint32_t* __restrict__ rng0,
-                            float4* __restrict__ rays) {
+                            float4* __restrict__ rays, uint32_t* __restrict__ cnt, uint32_t cnt_words) {
   grid_wait();
+  // the levels' queues and ray counts (a memset between two dependent launches
+  // would cost both their head starts)
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < cnt_words; i += blockDim.x) cnt[i] = 0u;
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < npix; q += gridDim.x * blockDim.x) {
     const uint32_t pix = pix0 + q;
     const uint32_t x = pix % Wd, y = pix / Wd;
@@ -633,10 +637,9 @@ cudaError_t launch_render_wave(const DeviceScene& S, const Cam& cam, uint32_t de
       for (uint32_t s0 = 0; s0 < spp; s0 += ns_pass) {
         const uint32_t ns = std::min(ns_pass, spp - s0);
         const uint32_t np = q * ns;
-        if ((e2 = cudaMemsetAsync(B.cnt, 0, 16 * ((size_t)depth + 1), cs)) != cudaSuccess) return e2;
         const uint32_t gb = std::min<uint32_t>(sms * 8, (q + 255) / 256);
         if ((e2 = launch_dependent(k_wave_seed, gb, 256, 0, cs, cam, rs, accum, Wd, pix0, q, ns, per_path, B.rng0,
-                                   B.rays[0])) != cudaSuccess)
+                                   B.rays[0], B.cnt, 4u * (depth + 1u))) != cudaSuccess)
           return e2;
         for (uint32_t l = 0; l < depth; ++l) {
           const float4* r = B.rays[l & 1u];
