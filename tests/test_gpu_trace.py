@@ -657,7 +657,7 @@ def test_shared_drain_is_sequential(rt, cuda, scene, n):
 
 
 @pytest.mark.parametrize("n", [1_572_863, 1_572_864, 2_000_001])
-def test_sorted_order_same_hits(rt, cuda, n):
+def test_reorder_at_its_line(rt, cuda, n):
     """On a tree beyond L2 a sorted batch is reordered from 1,572,864 rays on; hits do not change."""
     tris = rt.gen_soup(33, 0, 1_500_000, 1.0, 0.002)
     rays = rt.gen_rays(33, 0, n, 1.0, 1e-4, float("inf"))
