@@ -225,28 +225,42 @@ rt_status rt_stream_release(void* stream) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e, "rt_stream_release: cudaGetDevice");
-  trim_build_scratch(dev);
   Workspace* w = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_ws_mu);
     auto it = g_ws.find(std::make_pair(dev, st));
-    if (it == g_ws.end()) return RT_OK;
-    w = it->second;
-    g_ws.erase(it);
+    if (it != g_ws.end()) {
+      w = it->second;
+      g_ws.erase(it);
+    }
+  }
+  if (!w) {  // device builds take no workspace
+    if (!holds_build_scratch(dev)) return RT_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return RT_OK;  // a capture owns its scratch, and must not be waited for
+    }
   }
   // the library's work on the stream (and on its helper streams) ends first
   e = cudaStreamSynchronize(st);
-  for (cudaStream_t h : {w->copy_in, w->copy_out, w->trace2})
-    if (h) {
-      const cudaError_t e2 = cudaStreamSynchronize(h);
-      if (e == cudaSuccess) e = e2;
-      cudaStreamDestroy(h);
-    }
-  for (cudaEvent_t ev : w->ev)
-    if (ev) cudaEventDestroy(ev);
-  for (void* p : {static_cast<void*>(w->counters), w->stage, w->sort, w->wave})
-    if (p) cudaFree(p);
-  delete w;
+  if (w) {
+    for (cudaStream_t h : {w->copy_in, w->copy_out, w->trace2})
+      if (h) {
+        const cudaError_t e2 = cudaStreamSynchronize(h);
+        if (e == cudaSuccess) e = e2;
+        cudaStreamDestroy(h);
+      }
+    for (cudaEvent_t ev : w->ev)
+      if (ev) cudaEventDestroy(ev);
+    for (void* p : {static_cast<void*>(w->counters), w->stage, w->sort, w->wave})
+      if (p) cudaFree(p);
+    delete w;
+  }
+  // after the synchronisation: until then a build's scratch counts as in use,
+  // and would stay in the pool when the build ends
+  const cudaError_t e2 = trim_build_scratch(dev);
+  if (e == cudaSuccess) e = e2;
   return e == cudaSuccess ? RT_OK : cuda_fail(e, "rt_stream_release");
 }
 

@@ -1130,10 +1130,15 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
 
 }  // namespace
 
-void trim_build_scratch(int dev) {
+bool holds_build_scratch(int dev) {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  return g_pools.find(dev) != g_pools.end();
+}
+
+cudaError_t trim_build_scratch(int dev) {
   std::lock_guard<std::mutex> lk(g_pool_mu);
   auto it = g_pools.find(dev);
-  if (it != g_pools.end()) cudaMemPoolTrimTo(it->second, 0);
+  return it == g_pools.end() ? cudaSuccess : cudaMemPoolTrimTo(it->second, 0);
 }
 
 }  // namespace rtgb

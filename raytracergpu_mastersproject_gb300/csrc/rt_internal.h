@@ -268,7 +268,8 @@ cudaError_t launch_resolve(const float* accum, uint32_t w, uint32_t h, uint32_t 
 int device_sm_count();
 uint32_t spread_warps();  // see trace.cu
 // GPU LBVH build (gpu_build.cu)
-void trim_build_scratch(int dev);  // gives back the scratch kept between builds
+bool holds_build_scratch(int dev);        // whether a build has made the pool its scratch comes from
+cudaError_t trim_build_scratch(int dev);  // gives back the scratch kept between builds
 size_t device_build_scratch_bytes(uint32_t n);
 cudaError_t launch_device_build(const RtTriangle64* tris, uint32_t nt, const RtSphere32* sph, uint32_t ns,
                                 uint32_t mode, RtBVHNode40* nodes, void* scratch, cudaStream_t st);

@@ -166,3 +166,28 @@ def test_device_build_long_lists(rt, cuda, part):
     for v, d in (("v0", (-1, 0, 0)), ("v1", (0.5, 1, 0)), ("v2", (0.5, -1, 0))):
         t[v][:, :3] = centre + np.float32(1e-5) * np.array(d, np.float32)
     assert np.array_equal(device_build(rt, cuda, t).view(np.uint8), rt.build_bvh(t).view(np.uint8))
+
+
+@pytest.mark.parametrize("traced", [False, True], ids=["builds_only", "with_a_workspace"])
+def test_release_waits_for_the_build(rt, cuda, traced):
+    """rt_stream_release straight after a build, which is still running: its scratch (86 MB) goes back too, also on
+    a stream that has no workspace."""
+    tris = rt.gen_soup(14, 0, 4_194_304, 1.0, 0.002)
+    d_t = cuda.from_numpy(tris.view(np.uint8)).cuda()
+    d_n = cuda.zeros((2 * len(tris) - 1) * 40, dtype=cuda.uint8, device="cuda")
+    rays = cuda.zeros(32, dtype=cuda.uint8, device="cuda")
+    hits = cuda.zeros(8, dtype=cuda.uint8, device="cuda")
+    stream = cuda.cuda.Stream()
+    with rt.Scene(tris[:100]) as sc:
+        for turn in range(2):
+            cuda.cuda.synchronize()
+            if traced:
+                sc.trace(rays, hits, n=1, stream=stream)
+            rt.build_bvh_device(d_t, len(tris), d_nodes=d_n, stream=stream)
+            rt.release_stream(stream)
+            cuda.cuda.synchronize()
+            if turn == 0:  # whatever is kept from builds before this test
+                rt.release_stream()
+                free = cuda.cuda.mem_get_info()[0]
+    assert free - cuda.cuda.mem_get_info()[0] <= 4 << 20
+    assert np.array_equal(d_n.cpu().numpy(), rt.build_bvh(tris).view(np.uint8).ravel())
