@@ -17,6 +17,7 @@
 //   k_mid, k_last,   the same for the nodes above k_tree's blocks
 //   k_top
 #include <cooperative_groups.h>
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -1093,22 +1094,43 @@ namespace rtgb {
 namespace {
 
 // Scratch of device builds comes from a pool of the library's own, one per
-// device: the device's default pool gives its memory back at every
+// context: the device's default pool gives its memory back at every
 // synchronisation, and mapping it again cost a build after one 180 us (20,482
 // triangles, build and wait: 247 us, 80 us with the pool).  It keeps at most
 // kKeepBytes between builds -- scratch for 7 M primitives -- and
 // rt_stream_release hands that back.  Allocation and release are ordered on the
 // caller's stream, as before.
+//
+// A pool goes with its context, and a later one may come at the same address
+// (cudaDeviceReset); context ids are never used again, so a pool is found by the
+// id alone.
 constexpr uint64_t kKeepBytes = 256ull << 20;
 std::mutex g_pool_mu;
-std::map<int, cudaMemPool_t> g_pools;
+std::map<unsigned long long, cudaMemPool_t> g_pools;
+
+cudaError_t context_id(int dev, unsigned long long* id) {
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static const GetId get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &r);
+    return e == cudaSuccess && r == cudaDriverEntryPointSuccess ? reinterpret_cast<GetId>(f) : nullptr;
+  }();
+  if (!get) return cudaErrorNotSupported;
+  if (get(nullptr, id) == CUDA_SUCCESS) return cudaSuccess;
+  const cudaError_t e = cudaSetDevice(dev);  // a thread's first call, or one after a reset
+  if (e != cudaSuccess) return e;
+  return get(nullptr, id) == CUDA_SUCCESS ? cudaSuccess : cudaErrorDeviceUninitialized;
+}
 
 cudaError_t scratch_pool(cudaMemPool_t* out) {
   int dev = 0;
+  unsigned long long id = 0;
   cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = context_id(dev, &id);
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  auto it = g_pools.find(dev);
+  auto it = g_pools.find(id);
   if (it == g_pools.end()) {
     cudaMemPoolProps props;
     std::memset(&props, 0, sizeof(props));
@@ -1122,23 +1144,32 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
       cudaMemPoolDestroy(pool);
       return e;
     }
-    it = g_pools.emplace(dev, pool).first;
+    it = g_pools.emplace(id, pool).first;
   }
   *out = it->second;
   return cudaSuccess;
 }
 
-}  // namespace
-
-bool holds_build_scratch(int dev) {
+// The current context's pool; nullptr if no build has made one.
+cudaMemPool_t existing_pool(int dev) {
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (g_pools.empty()) return nullptr;
+  }
+  unsigned long long id = 0;
+  if (context_id(dev, &id) != cudaSuccess) return nullptr;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  return g_pools.find(dev) != g_pools.end();
+  auto it = g_pools.find(id);
+  return it == g_pools.end() ? nullptr : it->second;
 }
 
+}  // namespace
+
+bool holds_build_scratch(int dev) { return existing_pool(dev) != nullptr; }
+
 cudaError_t trim_build_scratch(int dev) {
-  std::lock_guard<std::mutex> lk(g_pool_mu);
-  auto it = g_pools.find(dev);
-  return it == g_pools.end() ? cudaSuccess : cudaMemPoolTrimTo(it->second, 0);
+  const cudaMemPool_t pool = existing_pool(dev);
+  return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
 }
 
 }  // namespace rtgb

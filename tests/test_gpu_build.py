@@ -2,11 +2,22 @@
 of the oracle's transcription of the six S1 passes (ModelSpaceToWorldSpace.comp
 to ConstructAABBsOfInternalNodes.comp), and of the host build."""
 import itertools
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+ROOT = Path(__file__).resolve().parent.parent
+
+
+def run_child(script):
+    """The script in a process of its own (argv: the repository's root)."""
+    r = subprocess.run([sys.executable, "-c", script, str(ROOT)], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-3000:]
 
 
 def device_build(rt, torch, tris, spheres=None, mode=0):
@@ -191,3 +202,33 @@ def test_release_waits_for_the_build(rt, cuda, traced):
                 free = cuda.cuda.mem_get_info()[0]
     assert free - cuda.cuda.mem_get_info()[0] <= 4 << 20
     assert np.array_equal(d_n.cpu().numpy(), rt.build_bvh(tris).view(np.uint8).ravel())
+
+
+RESET = r"""
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import raytracergpu_mastersproject_gb300 as rt
+L, runtime = rt.lib(), C.CDLL("/usr/local/cuda/lib64/libcudart.so")
+L.rt_device_alloc.argtypes = [C.c_size_t, C.POINTER(C.c_void_p)]
+L.rt_copy.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
+tris = rt.gen_soup(3, 0, 5000, 1.0, 0.01)
+want = rt.build_bvh(tris).view(np.uint8).ravel()
+for turn in range(3):
+    d_t, d_n = C.c_void_p(), C.c_void_p()
+    assert L.rt_device_alloc(tris.nbytes, C.byref(d_t)) == 0 and L.rt_device_alloc(want.nbytes, C.byref(d_n)) == 0
+    assert L.rt_copy(d_t.value, tris.ctypes.data, tris.nbytes, None) == 0
+    assert L.rt_build_bvh_device(d_t.value, len(tris), None, 0, 0, d_n.value, None) == 0, L.rt_last_error_string()
+    got = np.zeros_like(want)
+    assert L.rt_copy(got.ctypes.data, d_n.value, got.nbytes, None) == 0 and L.rt_stream_wait(None, 10.0) == 0
+    assert np.array_equal(got, want)
+    if turn == 1:
+        assert L.rt_stream_release(None) == 0
+    assert runtime.cudaDeviceReset() == 0
+assert L.rt_stream_release(None) == 0  # nothing of the present context to give back
+"""
+
+
+def test_device_build_after_a_device_reset(cuda):
+    """The pool of the builds' scratch belongs to a context: a build after cudaDeviceReset takes a new one."""
+    run_child(RESET)
