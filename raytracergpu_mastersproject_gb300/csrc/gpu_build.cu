@@ -1108,6 +1108,14 @@ constexpr uint64_t kKeepBytes = 256ull << 20;
 std::mutex g_pool_mu;
 std::map<unsigned long long, cudaMemPool_t> g_pools;
 
+// Lets the calling thread make and trim the pool while it captures a stream: a
+// capture refuses both otherwise, and is lost, although neither is part of it.
+struct AllowInCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  AllowInCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~AllowInCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 cudaError_t context_id(int dev, unsigned long long* id) {
   using GetId = CUresult (*)(CUcontext, unsigned long long*);
   static const GetId get = [] {
@@ -1132,6 +1140,7 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
   std::lock_guard<std::mutex> lk(g_pool_mu);
   auto it = g_pools.find(id);
   if (it == g_pools.end()) {
+    const AllowInCapture allow;
     cudaMemPoolProps props;
     std::memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -1169,6 +1178,7 @@ bool holds_build_scratch(int dev) { return existing_pool(dev) != nullptr; }
 
 cudaError_t trim_build_scratch(int dev) {
   const cudaMemPool_t pool = existing_pool(dev);
+  const AllowInCapture allow;
   return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
 }
 

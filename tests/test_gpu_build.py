@@ -232,3 +232,32 @@ assert L.rt_stream_release(None) == 0  # nothing of the present context to give 
 def test_device_build_after_a_device_reset(cuda):
     """The pool of the builds' scratch belongs to a context: a build after cudaDeviceReset takes a new one."""
     run_child(RESET)
+
+
+CAPTURE = r"""
+import sys
+import numpy as np, torch
+sys.path.insert(0, sys.argv[1])
+import raytracergpu_mastersproject_gb300 as rt
+for n in (5_000, 20_482, 300_000):  # one cluster, one group of tree blocks, several
+    soups = [rt.gen_soup(20 + k, 0, n, 1.0, 0.01) for k in range(2)]
+    want = [rt.build_bvh(t).view(np.uint8).ravel() for t in soups]
+    d_s = [torch.from_numpy(t.view(np.uint8)).cuda() for t in soups]
+    d_t, d_n = d_s[0].clone(), torch.zeros((2 * n - 1) * 40, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        rt.build_bvh_device(d_t, n, d_nodes=d_n, stream=torch.cuda.current_stream())
+    for k in (0, 1, 0):
+        d_t.copy_(d_s[k])
+        d_n.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(d_n.cpu().numpy(), want[k]), (n, k)
+"""
+
+
+def test_device_build_in_a_captured_graph(cuda):
+    """A captured build, the process's first one among them, replays on what the triangles are by then."""
+    run_child(CAPTURE)
