@@ -131,8 +131,14 @@ __global__ void __launch_bounds__(THREADS, MINB)
 // so the leaf code, which some lane needs in nearly every iteration, and the
 // loop's own work run less often (four is the default: config 3 13.24 ->
 // 11.78 ms per step against one).
+//
+// SPHERES: the scene has spheres, and lanes finish their own rays.  The shared
+// drain takes triangles alone: with spheres its launches could run for ever
+// (more rays than lanes, or many launches), and a ray whose hit is NaN -- a
+// sphere's root for a direction of length 0, or of products beyond binary32,
+// which counts as a hit as in the reference -- depends on its visiting order.
 template <bool ANY, int STACK, int THREADS, int MINB, bool STATS, bool RAW = false, int RING = 0, bool MT = false,
-          int TILE = 0, int VISITS = 1>
+          int TILE = 0, int VISITS = 1, bool SPHERES = false>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_trace_step(DeviceScene S, const float4* __restrict__ rays, uint32_t n, uint2* __restrict__ hits,
                  uint32_t* __restrict__ counter, int refill, unsigned long long* __restrict__ stats,
@@ -141,7 +147,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   using Stk = typename std::conditional<(RING > 0), dev::RingStack<(RING > 0 ? RING : 1), THREADS, dev::StepEntry>,
                                         dev::LocalStackT<dev::StepEntry>>::type;
   // The counting kernels count the sequential traversal.
-  constexpr bool kDrain = !STATS && RING == 16;
+  constexpr bool kDrain = !STATS && !SPHERES && RING == 16;
   Stk stk;
   if constexpr (RING > 0) {
     __shared__ dev::StepEntry ring[RING * THREADS];
@@ -290,6 +296,8 @@ struct Variant {
   bool drain;  // 4-wide trees end in the shared drain (step loop with the ring)
   TraceKernel k[2][2][2][2];  // [stats][wide][any][big stack]
   int blocks_per_sm[2][2][2][2];
+  TraceKernel with_spheres[2][2];  // of a shape with the drain: [any][big stack]
+  int with_spheres_bps[2][2];
 };
 
 template <int T, int M, bool ST>
@@ -319,6 +327,14 @@ Variant make_variant() {
   v.threads = T;
   v.minb = M;
   v.drain = STEP && RING == 16;
+  if constexpr (STEP && RING == 16) {
+    v.with_spheres[0][0] = k_trace_step<false, 64, T, M, false, false, RING, false, 0, VISITS, true>;
+    v.with_spheres[0][1] = k_trace_step<false, 192, T, M, false, false, RING, false, 0, VISITS, true>;
+    v.with_spheres[1][0] = k_trace_step<true, 64, T, M, false, false, RING, false, 0, VISITS, true>;
+    v.with_spheres[1][1] = k_trace_step<true, 192, T, M, false, false, RING, false, 0, VISITS, true>;
+  }
+  for (auto& a : v.with_spheres_bps)
+    for (int& b : a) b = -1;
   if constexpr (STEP) {
     fill_step_variant<T, M, false, RING, VISITS>(v);
     fill_step_variant<T, M, true, RING, VISITS>(v);
@@ -358,6 +374,8 @@ constexpr int kNumVariants = sizeof(g_variants) / sizeof(g_variants[0]);
 struct MtKernels {
   TraceKernel k[2][2][2];
   int blocks_per_sm[2][2][2];
+  TraceKernel with_spheres[2][2];  // [any][big stack]
+  int with_spheres_bps[2][2];
 };
 MtKernels g_mt = {{{{k_trace<false, 64, 128, 10, 2, false, true>, k_trace<false, 128, 128, 10, 2, false, true>},
                     {k_trace<true, 64, 128, 10, 2, false, true>, k_trace<true, 128, 128, 10, 2, false, true>}},
@@ -365,33 +383,44 @@ MtKernels g_mt = {{{{k_trace<false, 64, 128, 10, 2, false, true>, k_trace<false,
                      k_trace_step<false, 192, 128, 10, false, false, 16, true, 0, kDefaultVisits>},
                     {k_trace_step<true, 64, 128, 10, false, false, 16, true, 0, kDefaultVisits>,
                      k_trace_step<true, 192, 128, 10, false, false, 16, true, 0, kDefaultVisits>}}},
-                  {{{-1, -1}, {-1, -1}}, {{-1, -1}, {-1, -1}}}};
+                  {{{-1, -1}, {-1, -1}}, {{-1, -1}, {-1, -1}}},
+                  {{k_trace_step<false, 64, 128, 10, false, false, 16, true, 0, kDefaultVisits, true>,
+                    k_trace_step<false, 192, 128, 10, false, false, 16, true, 0, kDefaultVisits, true>},
+                   {k_trace_step<true, 64, 128, 10, false, false, 16, true, 0, kDefaultVisits, true>,
+                    k_trace_step<true, 192, 128, 10, false, false, 16, true, 0, kDefaultVisits, true>}},
+                  {{-1, -1}, {-1, -1}}};
 
 // The default launch shape (128 threads, 10 blocks per SM, 16-entry shared
 // ring, four node visits per iteration) at every tuned stack capacity and
 // staging tile (closest and any hit):
-// [any][kTunedStacks index][kTunedTiles index].
-template <bool ANY, int STACK>
+// [spheres][any][kTunedStacks index][kTunedTiles index].
+template <bool ANY, int STACK, bool SPHERES>
 void fill_tuned_row(TraceKernel* row) {
-  row[0] = k_trace_step<ANY, STACK, 128, 10, false, false, 16, false, 0, kDefaultVisits>;
-  row[1] = k_trace_step<ANY, STACK, 128, 10, false, false, 16, false, 16, kDefaultVisits>;
-  row[2] = k_trace_step<ANY, STACK, 128, 10, false, false, 16, false, 64, kDefaultVisits>;
+  row[0] = k_trace_step<ANY, STACK, 128, 10, false, false, 16, false, 0, kDefaultVisits, SPHERES>;
+  row[1] = k_trace_step<ANY, STACK, 128, 10, false, false, 16, false, 16, kDefaultVisits, SPHERES>;
+  row[2] = k_trace_step<ANY, STACK, 128, 10, false, false, 16, false, 64, kDefaultVisits, SPHERES>;
 }
 struct TunedKernels {
-  TraceKernel k[2][4][3];
-  int bps[2][4][3];
+  TraceKernel k[2][2][4][3];
+  int bps[2][2][4][3];
+  template <bool SPHERES>
+  void fill() {
+    fill_tuned_row<false, 48, SPHERES>(k[SPHERES][0][0]);
+    fill_tuned_row<false, 64, SPHERES>(k[SPHERES][0][1]);
+    fill_tuned_row<false, 96, SPHERES>(k[SPHERES][0][2]);
+    fill_tuned_row<false, 192, SPHERES>(k[SPHERES][0][3]);
+    fill_tuned_row<true, 48, SPHERES>(k[SPHERES][1][0]);
+    fill_tuned_row<true, 64, SPHERES>(k[SPHERES][1][1]);
+    fill_tuned_row<true, 96, SPHERES>(k[SPHERES][1][2]);
+    fill_tuned_row<true, 192, SPHERES>(k[SPHERES][1][3]);
+  }
   TunedKernels() {
-    fill_tuned_row<false, 48>(k[0][0]);
-    fill_tuned_row<false, 64>(k[0][1]);
-    fill_tuned_row<false, 96>(k[0][2]);
-    fill_tuned_row<false, 192>(k[0][3]);
-    fill_tuned_row<true, 48>(k[1][0]);
-    fill_tuned_row<true, 64>(k[1][1]);
-    fill_tuned_row<true, 96>(k[1][2]);
-    fill_tuned_row<true, 192>(k[1][3]);
+    fill<false>();
+    fill<true>();
     for (auto& a : bps)
       for (auto& b : a)
-        for (int& c : b) c = -1;
+        for (auto& c : b)
+          for (int& d : c) d = -1;
   }
 };
 TunedKernels g_tuned;
@@ -448,17 +477,22 @@ cudaError_t launch_trace_tuned(const DeviceScene& S, const RtRay* rays, uint32_t
   TraceKernel k = mt ? g_mt.k[wide][any][big] : v.k[st][wide][any][big];
   const int threads = mt ? 128 : v.threads;
   int* slot = mt ? &g_mt.blocks_per_sm[wide][any][big] : &v.blocks_per_sm[st][wide][any][big];
+  // these kernels hand out their first rays by position (see k_trace_step)
+  const bool spheres = S.n_spheres != 0u;
+  const bool drain = wide && !stats && (mt || v.drain) && !spheres;
+  if (wide && !stats && (mt || v.drain) && spheres) {
+    k = mt ? g_mt.with_spheres[any][big] : v.with_spheres[any][big];
+    slot = mt ? &g_mt.with_spheres_bps[any][big] : &v.with_spheres_bps[any][big];
+  }
   if (!stats && (tune.stack != 0 || tune.tile != 0)) {
     if (!tuning_supported(tune, S.width, S.stack_need, flags)) return cudaErrorInvalidValue;
     const int si = tune.stack == 0 ? (big ? 3 : 1) : tuned_index(kTunedStacks, 4, tune.stack);
     const int ti = tuned_index(kTunedTiles, 3, tune.tile);
-    k = g_tuned.k[any][si][ti];
-    slot = &g_tuned.bps[any][si][ti];
+    k = g_tuned.k[spheres][any][si][ti];
+    slot = &g_tuned.bps[spheres][any][si][ti];
   }
   int bps = 0;
   if (cudaError_t e = cached_blocks_per_sm(slot, k, threads, &bps); e != cudaSuccess) return e;
-  // these kernels hand out their first rays by position (see k_trace_step)
-  const bool drain = wide && !stats && (mt || v.drain);
   uint64_t blocks = (uint64_t)device_sm_count() * (uint64_t)bps * (uint64_t)std::max(1, tune.grid_scale) / 100u;
   uint64_t needed = ((uint64_t)n + threads - 1) / threads;
   if (drain) {  // few rays: a ray per warp at least, over up to `spread` warps
@@ -509,20 +543,17 @@ cudaError_t launch_trace_raw(const DeviceScene& S, const float4* rays, uint32_t 
   // node visits per iteration of the bounce queries (RT_TRACE_RAW_VISITS, 1-4)
   // (config 2 extended: 3.44 against 3.51 ms per frame with two than one)
   static const int visits = std::min(4, std::max(1, env_int("RT_TRACE_RAW_VISITS", 2)));
-  const int k = (big ? 1 : 0) | (stats ? 2 : 0) | ((visits - 1) << 2);
-  static int bps[16] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
-  static const TraceKernel table[16] = {
-      k_trace_step<false, 64, T, M, false, true, R>,         k_trace_step<false, 192, T, M, false, true, R>,
-      k_trace_step<false, 64, T, M, true, true, R>,          k_trace_step<false, 192, T, M, true, true, R>,
-      k_trace_step<false, 64, T, M, false, true, R, false, 0, 2>, k_trace_step<false, 192, T, M, false, true, R, false, 0, 2>,
-      k_trace_step<false, 64, T, M, true, true, R, false, 0, 2>,  k_trace_step<false, 192, T, M, true, true, R, false, 0, 2>,
-      k_trace_step<false, 64, T, M, false, true, R, false, 0, 3>, k_trace_step<false, 192, T, M, false, true, R, false, 0, 3>,
-      k_trace_step<false, 64, T, M, true, true, R, false, 0, 3>,  k_trace_step<false, 192, T, M, true, true, R, false, 0, 3>,
-      k_trace_step<false, 64, T, M, false, true, R, false, 0, 4>, k_trace_step<false, 192, T, M, false, true, R, false, 0, 4>,
-      k_trace_step<false, 64, T, M, true, true, R, false, 0, 4>,  k_trace_step<false, 192, T, M, true, true, R, false, 0, 4>};
-  TraceKernel kern = table[k];
+  const int k = (big ? 1 : 0) | (stats ? 2 : (S.n_spheres ? 4 : 0));
+  static int bps[4][6] = {{-1, -1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1, -1}};
+#define RT_RAW_ROW(V)                                                                                                  \
+  {k_trace_step<false, 64, T, M, false, true, R, false, 0, V>,       k_trace_step<false, 192, T, M, false, true, R, false, 0, V>, \
+   k_trace_step<false, 64, T, M, true, true, R, false, 0, V>,        k_trace_step<false, 192, T, M, true, true, R, false, 0, V>,  \
+   k_trace_step<false, 64, T, M, false, true, R, false, 0, V, true>, k_trace_step<false, 192, T, M, false, true, R, false, 0, V, true>}
+  static const TraceKernel table[4][6] = {RT_RAW_ROW(1), RT_RAW_ROW(2), RT_RAW_ROW(3), RT_RAW_ROW(4)};
+#undef RT_RAW_ROW
+  TraceKernel kern = table[visits - 1][k];
   int per_sm = 0;
-  if (cudaError_t e = cached_blocks_per_sm(&bps[k], kern, T, &per_sm); e != cudaSuccess) return e;
+  if (cudaError_t e = cached_blocks_per_sm(&bps[visits - 1][k], kern, T, &per_sm); e != cudaSuccess) return e;
   uint64_t blocks = (uint64_t)device_sm_count() * (uint64_t)per_sm;
   if (n != 0xFFFFFFFFu)
     blocks = std::min<uint64_t>(blocks, std::max<uint64_t>(((uint64_t)n + T - 1) / T,

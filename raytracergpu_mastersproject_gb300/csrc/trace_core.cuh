@@ -664,18 +664,16 @@ constexpr int kMinIdleDrain = 8;
 template <int STACK, bool MT, class Stk>
 __device__ __forceinline__ bool drain_step(const DeviceScene& S, Trav& s, Stk& stk) {
   const uint32_t ref = s.node;
-  if (is_leaf(ref) && (ref & kSphereBit)) {
-    leaf_visit<false, MT>(S, s, ref);
-    s.node = stk.pop(s);
-    return true;
-  }
   const bool inner = is_inner(ref);
+  const bool none = !inner && (ref & kSphereBit);  // an unused child slot: no primitive, a record of zeros misses
   const uint32_t at = inner ? ref : ref & kSlotMask;
-  if (chk(S.check, inner ? at >= S.n_inner : at >= S.n_tris, inner ? kChkNode : kChkTri, at)) return false;
+  if (chk(S.check, !none && (inner ? at >= S.n_inner : at >= S.n_tris), inner ? kChkNode : kChkTri, at)) return false;
   const void* base = inner ? S.inner : S.tris;
-  float4 a, b, c, d;
-  ldg8(base, 2u * at, a, b);
-  ldg8(base, 2u * at + 1u, c, d);
+  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a, c = a, d = a;
+  if (!none) {
+    ldg8(base, 2u * at, a, b);
+    ldg8(base, 2u * at + 1u, c, d);
+  }
   if (inner)
     return visit_wide_stk<STACK>(S, s, stk, [&](const DeviceScene&, uint32_t, float4& h, float4& r, float4& qa, float4& qb) {
       h = a; r = b; qa = c; qb = d;
@@ -690,7 +688,7 @@ __device__ __forceinline__ bool drain_step(const DeviceScene& S, Trav& s, Stk& s
     s.best = kLeafBit | at;
   }
   // a leaf of more triangles: the rest is a leaf of its own
-  s.node = (ref >> kCountShift & 7u) ? ref - (1u << kCountShift) + 1u : stk.pop(s);
+  s.node = !none && (ref >> kCountShift & 7u) ? ref - (1u << kCountShift) + 1u : stk.pop(s);
   return true;
 }
 

@@ -435,3 +435,21 @@ def test_frame_in_a_captured_graph(rt, cuda, size):
                 g.replay()
                 side.synchronize()
                 assert cuda.equal(acc, want[0]) and cuda.equal(img, want[1])
+
+
+def test_spheres_in_a_large_frame(rt, orc, cuda):
+    """Sphere records in a frame whose queries have more rays than the grid has lanes (2 x 259,200 primary rays):
+    lanes finish their own rays there."""
+    tris, mats = lit_scene(rt)
+    sph = np.zeros(64, rt.SPHERE_DTYPE)
+    sph["center"][:, :3] = np.random.default_rng(5).uniform(-2.0, 2.0, (64, 3)).astype(np.float32)
+    sph["radius"] = np.float32(0.2)
+    ubo = rt.make_ubo((0.0, 0.5, 4.0), (0.0, 0.0, 0.0), fov=60.0, depth=4, random_state=9)
+    w, h = 960, 540
+    bg = (0.3, 0.4, 0.5)
+    with rt.Scene(tris, spheres=sph, materials=mats) as sc:
+        img = gpu_render(rt, cuda, sc, ubo, w, h, 1, shade_mode=rt.SHADE_EXTENDED, background=bg,
+                         trace_every_primary=True)
+        ref = oracle_render(orc, tris, sc.nodes(), mats, ubo, w, h, 1, spheres=sph, extended=True, background=bg)
+    assert rmse(img, ref) <= 1e-3
+    assert np.mean(img == ref) > 0.99

@@ -665,3 +665,30 @@ def test_reorder_at_its_line(rt, cuda, n):
         want = dev_trace(rt, cuda, sc, rays).view(np.uint64)
         assert np.array_equal(dev_trace(rt, cuda, sc, rays, sort=True).view(np.uint64), want)
         assert np.array_equal(sc.trace_host(rays, sort=True).view(np.uint64), want)
+
+
+@pytest.mark.parametrize("scene", ["spheres", "mixed", "nan"])
+@pytest.mark.parametrize("n", [1, 33, 5_001, 200_003, 1_000_003])
+def test_spheres_in_every_batch_size(rt, cuda, scene, n):
+    """Batches on scenes with spheres, below and above a ray per lane of the grid: bit for bit the hits of the
+    launch shape whose lanes keep their stacks in local memory.  "nan": a sphere's root is NaN for a direction of
+    length 0 and where products overflow, and counts as a hit; which candidate such a ray ends with depends on
+    its whole visiting order."""
+    g = np.random.default_rng(34)
+    sph = np.zeros(300 if scene == "nan" else 20_000, rt.SPHERE_DTYPE)
+    sph["center"][:, :3] = g.random((len(sph), 3)).astype(np.float32)
+    sph["radius"] = np.float32(0.1 if scene == "nan" else 0.01)
+    tris = rt.gen_soup(34, 0, {"spheres": 0, "mixed": 20_000, "nan": 4_000}[scene], 1.0, 0.02)
+    rays = rt.gen_rays(34, 0, n, 1.0, 1e-4, float("inf"))
+    if scene == "nan":
+        rays["org"][::2] = sph["center"][np.arange(len(rays[::2])) % 300, :3] + np.float32(0.01)
+        rays["dir"][::4] = 0.0
+        rays["dir"][2::4] *= np.float32(1e25)
+    with rt.Scene(tris, spheres=sph) as sc:
+        got = [dev_trace(rt, cuda, sc, rays, any_hit=a) for a in (False, True)]
+        sc.set_tuning(rt.TraceTuning(14, 5, 0, 0, 0.0))
+        want = [dev_trace(rt, cuda, sc, rays, any_hit=a) for a in (False, True)]
+    if scene == "nan":
+        assert np.isnan(want[0]["t"][0])
+    for g, w in zip(got, want):
+        assert np.array_equal(g.view(np.uint64), w.view(np.uint64))
