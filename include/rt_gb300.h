@@ -244,7 +244,7 @@ enum {
   RT_TRACE_ANY = 1,      /* any hit in [tmin, tmax] (occlusion) */
   RT_TRACE_SORT = 2,     /* or'ed in: trace the batch in an order bucketed by ray origin
                             (coherence) where that pays (a large batch on a tree beyond
-                            L2); hits are unchanged and still land in ray order.
+                            L2, a smaller one on binary nodes); hits are unchanged and still land in ray order.
                             Uses a per-stream device workspace of about 10 bytes per ray. */
   RT_TRACE_MT = 4        /* or'ed in (rt_trace, rt_trace_host): the Moller-Trumbore
                             ray-triangle test (J. Graphics Tools 2(1), 1997) in binary32

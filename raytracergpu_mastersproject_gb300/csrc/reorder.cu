@@ -112,7 +112,16 @@ __global__ void __launch_bounds__(kSortThreads) k_bucket_scatter(const uint16_t*
 // order / reordered: 1,048,576 triangles (102 MB of records, in L2) 100,003 rays
 // 179 / 210, 16 M rays 7,985 / 8,135; 2,097,152 (204 MB) 2 M rays 1,253 / 1,243,
 // 16 M rays 8,918 / 8,559; 4,194,304 (408 MB) 1 M rays 765 / 772, 2 M rays
-// 1,369 / 1,327, 16 M rays 9,754 / 8,978.
+// 1,369 / 1,327, 16 M rays 9,754 / 8,978.  Any hit crosses at the same sizes;
+// rays of a short interval later (4,194,304 triangles, 4 M rays 845 / 880).
+//
+// Binary trees gain earlier: a ray fetches three times the records, one after
+// the other, and a warp of one cell shares them in L1.  262,144 triangles (34 MB)
+// 150,000 rays 377 / 409, 300,000 565 / 556, 4 M 5,626 / 5,286; 4,194,304 (537 MB)
+// 150,000 620 / 711, 300,000 912 / 901, 4 M 8,750 / 7,154 (short intervals 1,800 /
+// 1,407).  Trees of a few MB cross later (10,000 triangles, 1.3 MB: 300,000 rays
+// 295 / 295, short 95 / 109, 600,000 508 / 486, 159 / 159; 2,000: 600,000 279 / 292,
+// 1.6 M 651 / 654), those within L1 not at all (200: 4 M rays 712 / 751).
 bool reorder_pays(const DeviceScene& S, uint32_t n) {
   static int cached = -1;
   int l2 = __atomic_load_n(&cached, __ATOMIC_RELAXED);
@@ -123,6 +132,9 @@ bool reorder_pays(const DeviceScene& S, uint32_t n) {
     __atomic_store_n(&cached, l2, __ATOMIC_RELAXED);
   }
   const uint64_t records = 64ull * S.n_inner + 64ull * S.n_tris;
+  if (S.width == 2)
+    return n >= (records > (8u << 20) ? 1u << 18 : records > (1u << 20) ? 1u << 19 : kMinReorderRays) &&
+           records > (128u << 10);
   return n >= kMinReorderRays && records > (uint64_t)l2;
 }
 

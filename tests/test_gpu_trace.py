@@ -692,3 +692,33 @@ def test_spheres_in_every_batch_size(rt, cuda, scene, n):
         assert np.isnan(want[0]["t"][0])
     for g, w in zip(got, want):
         assert np.array_equal(g.view(np.uint64), w.view(np.uint64))
+
+
+def reorder_scratch(rt, torch, scene, n, **kw):
+    """Device memory that a first sorted batch of n rays takes on a stream of its own beside an unsorted one's, and
+    whether the hits agree."""
+    rays = torch.from_numpy(rt.gen_rays(35, 0, n, 1.0, 1e-4, float("inf")).view(np.uint8)).cuda()
+    hits = [torch.zeros(n * 8, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    scene.trace(rays, hits[0], stream=stream, **kw)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    scene.trace(rays, hits[1], stream=stream, sort=True, **kw)
+    torch.cuda.synchronize()
+    used = free - torch.cuda.mem_get_info()[0]
+    rt.release_stream(stream)
+    return used, torch.equal(*hits)
+
+
+@pytest.mark.parametrize("width, tris, n, reordered",
+                         [(2, 80_000, 262_143, False), (2, 80_000, 262_144, True), (2, 20_000, 524_287, False),
+                          (2, 20_000, 524_288, True), (2, 2_000, 1_572_864, True), (2, 200, 2_000_000, False),
+                          (4, 80_000, 2_000_000, False)])
+def test_where_a_sorted_batch_is_reordered(rt, cuda, width, tris, n, reordered):
+    """The reorder takes about ten bytes a ray; where it does not pay it is not made.  Binary trees gain from it
+    long before 4-wide ones."""
+    with rt.Scene(rt.gen_soup(35, 0, tris, 1.0, 0.01), node_width=width) as sc:
+        for any_hit in (False, True):
+            used, same = reorder_scratch(rt, cuda, sc, n, any_hit=any_hit)
+            assert (used >= 2 << 20) == reordered and same
