@@ -16,6 +16,8 @@
 //                    atomicAdd, then place each ray at its range + its rank
 #include <cuda_runtime.h>
 
+#include <cstdlib>
+
 #include "rt_internal.h"
 
 namespace rtgb {
@@ -122,7 +124,15 @@ __global__ void __launch_bounds__(kSortThreads) k_bucket_scatter(const uint16_t*
 // 1,407).  Trees of a few MB cross later (10,000 triangles, 1.3 MB: 300,000 rays
 // 295 / 295, short 95 / 109, 600,000 508 / 486, 159 / 159; 2,000: 600,000 279 / 292,
 // 1.6 M 651 / 654), those within L1 not at all (200: 4 M rays 712 / 751).
+//
+// RT_TRACE_SORT_MIN_RAYS=n draws the line at n rays whatever the tree, for
+// batches that the rule above does not fit.
 bool reorder_pays(const DeviceScene& S, uint32_t n) {
+  static const long long line = [] {
+    const char* e = std::getenv("RT_TRACE_SORT_MIN_RAYS");
+    return e && *e ? std::atoll(e) : -1ll;
+  }();
+  if (line >= 0) return (long long)n >= line;
   static int cached = -1;
   int l2 = __atomic_load_n(&cached, __ATOMIC_RELAXED);
   if (l2 < 0) {

@@ -6,11 +6,18 @@ binary64 arbiter (oracle.arbitrate) accepts; matching hits must carry the
 bit-identical binary32 t.
 """
 import ctypes as C
+import os
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+# 0 or more: every sorted batch of at least so many rays is reordered (RT_TRACE_SORT_MIN_RAYS)
+SORT_LINE = int(os.environ.get("RT_TRACE_SORT_MIN_RAYS") or -1)
 
 
 def dev_trace(rt, torch, scene, rays, any_hit=False, sort=False):
@@ -718,7 +725,24 @@ def reorder_scratch(rt, torch, scene, n, **kw):
 def test_where_a_sorted_batch_is_reordered(rt, cuda, width, tris, n, reordered):
     """The reorder takes about ten bytes a ray; where it does not pay it is not made.  Binary trees gain from it
     long before 4-wide ones."""
+    if SORT_LINE >= 0:
+        reordered = n >= SORT_LINE
     with rt.Scene(rt.gen_soup(35, 0, tris, 1.0, 0.01), node_width=width) as sc:
         for any_hit in (False, True):
             used, same = reorder_scratch(rt, cuda, sc, n, any_hit=any_hit)
             assert (used >= 2 << 20) == reordered and same
+
+
+@pytest.mark.skipif(SORT_LINE >= 0, reason="this is the process it starts")
+@pytest.mark.parametrize("tests", [
+    "test_gpu_trace.py -k 'where_a_sorted or sorted_order or deep_stacks or degenerate_rays or mt_mode or autotune or "
+    "alignment or host_matches'", "test_gpu_fuzz.py -k scenes", "test_gpu_checks.py"])
+def test_sorted_batches_with_the_reorder(cuda, tests):
+    """The tests that ask for a sorted order, most on batches that would not be reordered by themselves, with every
+    batch reordered: awkward rays, deep stacks, every launch shape, host chunks, the checked build."""
+    name, *rest = tests.split(" -k ")
+    cmd = [sys.executable, "-m", "pytest", "-x", "-q", "-m", "gpu", str(Path(__file__).resolve().parent / name)]
+    cmd += ["-k", rest[0].strip("'")] if rest else []
+    r = subprocess.run(cmd, env=dict(os.environ, RT_TRACE_SORT_MIN_RAYS="1"), capture_output=True, text=True,
+                       timeout=900)
+    assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-3000:] + r.stderr[-1000:]
