@@ -746,3 +746,16 @@ def test_sorted_batches_with_the_reorder(cuda, tests):
     r = subprocess.run(cmd, env=dict(os.environ, RT_TRACE_SORT_MIN_RAYS="1"), capture_output=True, text=True,
                        timeout=900)
     assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-3000:] + r.stderr[-1000:]
+
+
+def test_host_chunks_are_reordered_on_both_streams(rt, cuda):
+    """8,000,001 host rays on a tree beyond L2: the chunks after the first, of 2 Mi and 4.9 M rays, are reordered at
+    the same time, each on its own stream and in its own half of the scratch."""
+    n = 8_000_001
+    rays = rt.gen_rays(36, 0, n, 1.0, 1e-4, float("inf"))
+    with rt.Scene(rt.gen_soup(36, 0, 1_500_000, 1.0, 0.002)) as sc:
+        for any_hit in (False, True):
+            want = dev_trace(rt, cuda, sc, rays, any_hit=any_hit).view(np.uint64)
+            for _ in range(2):
+                got = sc.trace_host(rays, any_hit=any_hit, sort=True)
+                assert np.array_equal(got.view(np.uint64), want)
