@@ -542,10 +542,10 @@ uint32_t rt_device_checks_compiled(void);
 rt_status rt_scene_device_checks(rt_scene* scene, uint32_t* bits, uint32_t* first_index);
 /* Frees the device workspace the library keeps for this stream on the current
  * device (work counters, ray staging, reorder and path-tracing scratch), after
- * the stream's work has finished, and the scratch kept between device BVH
- * builds (at most 256 MiB per device).  No call on the stream may run concurrently;
- * a later call on it allocates a new workspace.  No counterpart in the
- * reference. */
+ * the stream's work has finished, and the scratch that the current context keeps
+ * between device BVH builds (at most 256 MiB; scratch in use on other streams
+ * stays).  No call on the stream may run concurrently; a later call on it
+ * allocates a new workspace.  No counterpart in the reference. */
 rt_status rt_stream_release(void* stream);
 /* How many per-(device, stream) workspaces the library holds: each is created
  * with cudaMalloc the first time rt_trace, rt_trace_host, rt_trace_count or

@@ -307,7 +307,7 @@ class Scene:
     def trace(self, rays, hits, n: int | None = None, any_hit: bool = False, sort: bool = False, stream=None,
               mt: bool = False) -> None:
         """rays/hits: device tensors holding RtRay / RtHit records (stream-ordered).
-        sort: trace in an origin-bucketed order for coherence (same results).
+        sort: trace in an origin-bucketed order for coherence where that pays (same results).
         mt: the Moller-Trumbore triangle test instead of the reference's plane test."""
         if n is None:
             n = rays.numel() * rays.element_size() // RAY_DTYPE.itemsize

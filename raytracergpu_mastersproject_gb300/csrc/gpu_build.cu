@@ -564,10 +564,10 @@ __device__ __forceinline__ int delta_next(const uint32_t* __restrict__ codes, ui
 // A block of k_tree owns kLeaves consecutive leaves.  Splits inside it meet in
 // shared memory, and its records leave as whole lines.  The few nodes whose
 // parent reaches over an edge of the block go to a list, from which k_mid and
-// k_top climb on; climbing on through global slots in k_tree itself kept whole
-// blocks resident for one thread's chain of atomics.  The two replace a leaf pass, a pass of Karras
-// searches and a bottom-up pass with a global atomic and two 40-byte record
-// reads per node.  4,194,304 triangles: 666 us for those three; k_tree 311 us as
+// k_last or k_top climb on; climbing on through global slots in k_tree itself
+// kept whole blocks resident for one thread's chain of atomics.  They replace a
+// leaf pass, a pass of Karras searches and a bottom-up pass with a global atomic
+// and two 40-byte record reads per node.  4,194,304 triangles: 666 us for those three; k_tree 311 us as
 // one climb per thread, 260 with the climb cut in two, 195 with 8-byte stores,
 // padded rows and one box array (bound by issue; 518 MB read, most of it the
 // gather, and 289 MB written); k_top 65 us of serial atomics.
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(kLeaves) k_tree(const RtTriangle64* __restrict
       put(out_inner + 2u * j, x, y);
     }
   }
-  // The nodes k_mid climbs on from: those at the edges and the visitors that
+  // The nodes the next kernel climbs on from: those at the edges and the visitors that
   // met nobody in their shared slot.
   const uint32_t tag = slot[t];
   uint32_t mine = 0u;
@@ -941,8 +941,11 @@ __global__ void __launch_bounds__(kMidThreads) k_mid(uint32_t n, const uint32_t*
 }
 
 // The top of a tree of several groups: the nodes that k_mid's groups left, about
-// ten each, ranked by counting, in one block.  Leaves the work to k_top when they
-// are too many or some group's list was too long.
+// ten each, ranked by counting, in one block.  Leaves the work to k_top when some
+// group's list was too long.  They are never too many by themselves: they are one
+// more than the nodes that reach over an edge between groups, and over each of the
+// 47 edges of kLastGroups reach at most 36 (30 lengths of common prefix of two
+// codes, six of two positions of one code), less the shared ones.
 __device__ __forceinline__ bool fits_last(uint32_t num_next) { return num_next <= kMidItems; }
 
 __global__ void __launch_bounds__(kMidThreads) k_last(uint32_t n, const uint32_t* __restrict__ codes,
@@ -1097,8 +1100,8 @@ namespace {
 // context: the device's default pool gives its memory back at every
 // synchronisation, and mapping it again cost a build after one 180 us (20,482
 // triangles, build and wait: 247 us, 80 us with the pool).  It keeps at most
-// kKeepBytes between builds -- scratch for 7 M primitives -- and
-// rt_stream_release hands that back.  Allocation and release are ordered on the
+// kKeepBytes between builds -- scratch for 13 M primitives at 20.5 bytes each --
+// and rt_stream_release hands that back.  Allocation and release are ordered on the
 // caller's stream, as before.
 //
 // A pool goes with its context, and a later one may come at the same address

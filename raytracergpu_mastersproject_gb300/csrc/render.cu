@@ -465,14 +465,13 @@ __global__ void k_wave_seed(Cam cam, uint32_t random_state, float4* __restrict__
 // 2,770 instead of 2,864 us (2,809 with 4 blocks of 256).
 constexpr int kShadeThreads = 128, kShadeBlocks = 10;
 template <bool STATS>
-__global__ void __launch_bounds__(kShadeThreads, kShadeBlocks) k_wave_shade(DeviceScene S, uint32_t level, uint32_t depth, uint32_t n0, uint32_t npix, uint32_t ns,
-                             uint32_t per_path, uint32_t mode, float bgx, float bgy, float bgz,
-                             float4* __restrict__ color_of, float4* __restrict__ gatt_of,
-                             const uint32_t* __restrict__ rng0,
-                             const float4* __restrict__ rays, const uint32_t* __restrict__ list,
-                             const uint2* __restrict__ hits, float4* __restrict__ next_rays,
-                             uint32_t* __restrict__ next_list, uint32_t* __restrict__ cnt,
-                             uint32_t* __restrict__ status_word, unsigned long long* __restrict__ stats) {
+__global__ void __launch_bounds__(kShadeThreads, kShadeBlocks)
+    k_wave_shade(DeviceScene S, uint32_t level, uint32_t depth, uint32_t n0, uint32_t npix, uint32_t ns,
+                 uint32_t per_path, uint32_t mode, float bgx, float bgy, float bgz, float4* __restrict__ color_of,
+                 float4* __restrict__ gatt_of, const uint32_t* __restrict__ rng0, const float4* __restrict__ rays,
+                 const uint32_t* __restrict__ list, const uint2* __restrict__ hits, float4* __restrict__ next_rays,
+                 uint32_t* __restrict__ next_list, uint32_t* __restrict__ cnt, uint32_t* __restrict__ status_word,
+                 unsigned long long* __restrict__ stats) {
   grid_wait();
   const uint32_t n = level == 0 ? n0 : *reinterpret_cast<volatile uint32_t*>(cnt + 4u * level + 2u);
   if (STATS && level == 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stats[0], (unsigned long long)(per_path ? n0 : npix));

@@ -75,9 +75,9 @@ struct NvtxRange {
 // first on every path: from there on the one before it has ended and its writes
 // are visible.  Saves most of the gap between two dependent launches: a 317x179
 // preview of twelve kernels takes 97 us instead of 124 (84 without memsets between
-// them), a 1280x720 frame 2,744 instead of 2,771.  (Letting the next kernel's blocks in as soon as this one
-// has started, griddepcontrol.launch_dependents, holds places that the other
-// stream's blocks need: 105 and 2,964 us.)
+// them), a 1280x720 frame 2,744 instead of 2,771.  (Letting the next kernel's
+// blocks in as soon as this one has started, griddepcontrol.launch_dependents,
+// holds places that the other stream's blocks need: 105 and 2,964 us.)
 template <class... P, class... A>
 cudaError_t launch_dependent(void (*k)(P...), dim3 grid, uint32_t block, size_t smem, cudaStream_t st,
                              A&&... args) {

@@ -512,8 +512,8 @@ cudaError_t launch_trace_tuned(const DeviceScene& S, const RtRay* rays, uint32_t
   return cudaGetLastError();
 }
 
-// Warps over which a closest-hit step-loop launch spreads fewer rays than they
-// have lanes: eight per SM, two per scheduler, which still leaves every warp's
+// Warps over which a launch that ends in the shared drain spreads fewer rays than
+// they have lanes: eight per SM, two per scheduler, which still leaves every warp's
 // chain of fetches nearly to itself.  17 rays on 20,482 triangles take 12.3 us
 // so and 14.9 in one warp; a 317x179 preview's four bounce levels 124 against
 // 157 us (4 and 16 warps per SM: 124 and 121).

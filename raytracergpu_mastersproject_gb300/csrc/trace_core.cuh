@@ -592,8 +592,8 @@ __device__ __forceinline__ bool visit_wide_stk(const DeviceScene& S, Trav& s, St
 }
 
 // ------------------------------------------------------ shared drain ----
-// The end of a closest-hit launch, when the ray queue is empty: a warp's last
-// rays are finished by all of its lanes.  Free paths are exponentially
+// The end of a launch on triangles, closest or any hit, when the ray queue is
+// empty: a warp's last rays are finished by all of its lanes.  Free paths are exponentially
 // distributed, so a launch's longest rays visit many times the mean, and a
 // small launch lasted as long as its longest ray's chain of dependent fetches
 // with one lane of a warp at work.  Here a lane without work takes the bottom
